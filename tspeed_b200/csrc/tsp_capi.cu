@@ -23,6 +23,7 @@
 #include "tsp_tcfx.cuh"
 #include "tsp_dmma.cuh"
 #include "tsp_simt32.cuh"
+#include "tsp_rowring.cuh"
 
 namespace {
 
@@ -36,6 +37,12 @@ struct tsp_handle {
   int ne = 0, N = 0, Np = 0, R = 0, S = 1, nrcv = 0;
   long long nnzb = 0;
   int prec = TSP_PREC_FP64, op_kind = TSP_OP_EXPLICIT;
+  // Single-shot explicit FP64 / FP32 handles store symmetric operators once
+  // per face: stored block << 1 | transposed of each pattern entry (empty: the
+  // pattern's own order), the rows' references on the device, stored blocks.
+  std::vector<int> bref;
+  tsp::RowRefs* d_rows = nullptr;
+  long long nstored = 0;
   int bpitch = 0;  // column pitch of stored blocks: 2Np (one shot) or 2Np rounded up to 4 (batched)
   // Non-orthonormal basis (BoundaryAdapted): M_ref = L L^T (Cholesky). The
   // device works in the orthonormalised coordinates w = L^T u of every
@@ -455,14 +462,43 @@ int set_basis_mass(tsp_handle* h, int basis, const std::vector<double>& mass, co
 // Turns FP64 blocks B on the device (column-major, pitch pin; overwritten)
 // into L^-1 B L^-T in the handle's storage type at h->d_blocks.
 int fold_blocks(tsp_handle* h, double* d_in, int pin) {
-  tsp::k_fold_basis<<<unsigned(h->nnzb), 256, 0, h->stream>>>(d_in, pin, h->Np, h->d_lref_inv, 0, TSP_PREC_FP64, pin,
+  tsp::k_fold_basis<<<unsigned(h->nstored), 256, 0, h->stream>>>(d_in, pin, h->Np, h->d_lref_inv, 0, TSP_PREC_FP64, pin,
                                                              d_in, nullptr);
-  tsp::k_fold_basis<<<unsigned(h->nnzb), 256, 0, h->stream>>>(d_in, pin, h->Np, h->d_lref_inv, 1, h->prec, h->bpitch,
+  tsp::k_fold_basis<<<unsigned(h->nstored), 256, 0, h->stream>>>(d_in, pin, h->Np, h->d_lref_inv, 1, h->prec, h->bpitch,
                                                              h->d_blocks, h->d_bscale);
   cudaError_t ce = cudaGetLastError();
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
   if (ce != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("basis fold: ") + cudaGetErrorString(ce));
   return TSP_OK;
+}
+
+// Rows of block references for the ring kernel from the pattern and bref.
+int upload_rows(tsp_handle* h, const int* row_ptr, const int* col) {
+  std::vector<tsp::RowRefs> rows(h->ne);
+  for (int e = 0; e < h->ne; ++e)
+    for (int q = 0; q < 4; ++q) {
+      const int b = row_ptr[e] + q;
+      const bool in = b < row_ptr[e + 1];
+      rows[e].q[q].col = in ? col[b] : -1;
+      rows[e].q[q].ref = in ? h->bref[b] : -1;
+    }
+  int rc = upload(h, &h->d_rows, rows.data(), rows.size());
+  if (rc) return rc;
+  TSP_CUDA(h, cudaStreamSynchronize(h->stream));  // `rows` ends here
+  return TSP_OK;
+}
+
+// Single-shot handles with stored blocks advance by the ring kernel on
+// symmetric storage from 2Np = 30 on, FP64 ones from 2Np = 20 on. Below, a row
+// is so short that the ring kernel's work per row, not its bytes, sets the
+// time, and the register-streaming row kernel wins (40,000 triangles, us per
+// step, ring / rows: FP64 2Np = 12 85 / 37, 20 74 / 84, 30 117 / 327; FP32
+// 2Np = 20 65 / 50, 30 70 / 97). BF16 blocks are not multiples of the 16 bytes
+// of a bulk copy.
+constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 30); }
+bool uses_rowring(const tsp_handle* h) {
+  return h->S == 1 && h->op_kind == TSP_OP_EXPLICIT && h->prec != TSP_PREC_BF16 &&
+         rowring_size(h->R, h->prec == TSP_PREC_FP64);
 }
 
 int finish_create(tsp_handle* h) {
@@ -756,8 +792,47 @@ int launch_ksplit(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   return TSP_OK;
 }
 
+// Single-shot ring kernel: persistent, one team of four warps per CTA, launched with programmatic stream serialization so that a step's rings fill
+// while the previous step ends.
+template <int R, typename BT>
+int launch_rowring(tsp_handle* h, const tsp::StepParams& p0, cudaStream_t st) {
+  typedef tsp::RowRingCfg<R, BT> CF;
+  constexpr size_t smem = CF::smem_bytes();
+  static_assert(CF::CTAS >= 1 && CF::CTAS * (smem + 1024) <= 228 * 1024, "row ring kernel shared memory");
+  static unsigned long long configured = 0;
+  const unsigned long long bit = 1ull << (h->device & 63);
+  auto kern = tsp::k_step_rowring<R, BT>;
+  if (!(configured & bit)) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("row ring kernel smem: ") + cudaGetErrorString(e));
+    configured |= bit;
+  }
+  tsp::StepParams p = p0;
+  p.rows = h->d_rows;
+  p.nphys = int(h->nstored);
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(unsigned(std::min<long long>(p.ne, (long long)CF::CTAS * h->num_sms)));
+  lc.blockDim = dim3(CF::W * 32);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&lc, kern, p, h->d_err);
+  if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("row ring kernel: ") + cudaGetErrorString(e));
+  return TSP_OK;
+}
+
 template <int R>
 int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
+  if (h->d_rows) {
+    if constexpr (rowring_size(R, true))
+      if (h->prec == TSP_PREC_FP64) return launch_rowring<R, double>(h, p, st);
+    if constexpr (rowring_size(R, false))
+      if (h->prec == TSP_PREC_FP32) return launch_rowring<R, float>(h, p, st);
+  }
   if constexpr (R <= 56) {
     if (h->fx && (p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst)) return launch_fx<R>(h, p, st);
   }
@@ -812,18 +887,20 @@ int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   typedef tsp::RowTeam<R, double> RT;
   const long long teams = (long long)h->ne * p.S;
   const unsigned grid = unsigned((teams + RT::TEAMS_PER_CTA - 1) / RT::TEAMS_PER_CTA);
+  // Blocks at the batched kernels' pitch (several shots: single-vector
+  // products), or at 2Np (one shot, where the ring kernel does not apply).
   const bool padded = p.bpitch != R;
   switch (h->prec) {
     case TSP_PREC_FP64:
-      if (padded) tsp::k_step_rows<R, double, true><<<grid, RT::THREADS, 0, st>>>(p);
-      else tsp::k_step_rows<R, double, false><<<grid, RT::THREADS, 0, st>>>(p);
+      if (padded || R % 4 == 0) tsp::k_step_rows<R, double, true><<<grid, RT::THREADS, 0, st>>>(p);
+      else if constexpr (!rowring_size(R, true)) tsp::k_step_rows<R, double, false><<<grid, RT::THREADS, 0, st>>>(p);
       break;
     case TSP_PREC_FP32:
-      if (padded) tsp::k_step_rows<R, float, true><<<grid, RT::THREADS, 0, st>>>(p);
-      else tsp::k_step_rows<R, float, false><<<grid, RT::THREADS, 0, st>>>(p);
+      if (padded || R % 4 == 0) tsp::k_step_rows<R, float, true><<<grid, RT::THREADS, 0, st>>>(p);
+      else if constexpr (!rowring_size(R, false)) tsp::k_step_rows<R, float, false><<<grid, RT::THREADS, 0, st>>>(p);
       break;
     default:
-      if (padded) tsp::k_step_rows<R, __nv_bfloat16, true><<<grid, RT::THREADS, 0, st>>>(p);
+      if (padded || R % 4 == 0) tsp::k_step_rows<R, __nv_bfloat16, true><<<grid, RT::THREADS, 0, st>>>(p);
       else tsp::k_step_rows<R, __nv_bfloat16, false><<<grid, RT::THREADS, 0, st>>>(p);
       break;
   }
@@ -1134,6 +1211,8 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
   std::vector<int8_t> bface;
   tsp::bsr_pattern(P->ne, neigh.data(), &row_ptr, &col, &bface);
   h->nnzb = (long long)col.size();
+  h->nstored = h->nnzb;
+  if (uses_rowring(h)) h->nstored = tsp::symmetric_refs(P->ne, nedge.data(), row_ptr, col, bface, &h->bref);
   tsp::RefTables T = tsp::make_tables(P->N, P->basis);
   if (P->basis != TSP_BASIS_DUBINER && (rc = set_basis_mass(h, P->basis, T.M, T.Minv))) return create_error_from(h, rc);
 
@@ -1224,18 +1303,23 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
   const size_t esz = h->prec == TSP_PREC_FP64 ? 8 : (h->prec == TSP_PREC_FP32 ? 4 : 2);
   {
     void* blk = nullptr;
-    cudaError_t ce = pool_alloc(h, &blk, size_t(h->nnzb) * RRp * esz);
+    cudaError_t ce = pool_alloc(h, &blk, size_t(h->nstored) * RRp * esz);
     if (ce != cudaSuccess) {
-      fail(h, TSP_ERR_NOMEM, "operator blocks (" + std::to_string(size_t(h->nnzb) * RRp * esz) +
+      fail(h, TSP_ERR_NOMEM, "operator blocks (" + std::to_string(size_t(h->nstored) * RRp * esz) +
                                  " bytes) do not fit: " + cudaGetErrorString(ce));
       return create_error_from(h, TSP_ERR_NOMEM);
     }
     h->owned.push_back(blk);
     h->d_blocks = blk;
-    if (h->bpitch != h->R) TSP_CUDA(h, cudaMemsetAsync(blk, 0, size_t(h->nnzb) * RRp * esz, h->stream));
+    if (h->bpitch != h->R) TSP_CUDA(h, cudaMemsetAsync(blk, 0, size_t(h->nstored) * RRp * esz, h->stream));
   }
   if (h->prec == TSP_PREC_BF16 && (rc = dalloc(h, &h->d_bscale, size_t(h->nnzb)))) return create_error_from(h, rc);
+  int* d_bref = nullptr;
+  if (!h->bref.empty() && ((rc = upload_rows(h, row_ptr.data(), col.data())) ||
+                           (rc = upload(h, &d_bref, h->bref.data(), h->bref.size()))))
+    return create_error_from(h, rc);
   tsp::AssembleParams ap;
+  ap.ref = d_bref;
   ap.ne = h->ne;
   ap.N = h->N;
   ap.Np = h->Np;
@@ -1266,7 +1350,7 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
   if (!h->lref.empty()) {
     ap.prec = TSP_PREC_FP64;
     if (h->prec != TSP_PREC_FP64) {
-      if ((rc = dalloc(h, &d_tmp, size_t(h->nnzb) * h->R * h->R))) return create_error_from(h, rc);
+      if ((rc = dalloc(h, &d_tmp, size_t(h->nstored) * h->R * h->R))) return create_error_from(h, rc);
       ap.out = d_tmp;
       ap.pitch = h->R;
     }
@@ -1288,7 +1372,7 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
   }
   for (void* q : {(void*)d_neigh, (void*)d_nedge, (void*)d_bface, (void*)d_invJ, (void*)d_detJ, (void*)d_elen,
                   (void*)d_enrm, (void*)d_lam, (void*)d_mu, (void*)d_K, (void*)d_Ws, (void*)d_Wx, (void*)d_Ds,
-                  (void*)d_Dx})
+                  (void*)d_Dx, (void*)d_bref})
     dfree(h, q);
   if ((rc = finish_create(h))) return create_error_from(h, rc);
   *out = h;
@@ -1349,22 +1433,37 @@ int tsp_create_from_blocks(const tsp_block_problem* P, tsp_handle** out) {
   const int R = h->R;
   const size_t RR = size_t(R) * R;
   h->bpitch = block_pitch(R, h->S);
+  // The stored blocks, as entries of the pattern.
+  std::vector<int> stored;
+  if (uses_rowring(h)) {
+    int32_t n = 0;
+    tsp::symmetric_refs_of_blocks(P->ne, R, P->row_ptr, P->col, P->blocks, &h->bref, &n);
+    stored.resize(n);
+    for (int b = 0; b < P->nnzb; ++b)
+      if (!(h->bref[b] & 1)) stored[h->bref[b] >> 1] = b;
+    if ((rc = upload_rows(h, P->row_ptr, P->col))) return create_error_from(h, rc);
+  } else {
+    stored.resize(P->nnzb);
+    std::iota(stored.begin(), stored.end(), 0);
+  }
+  const int nst = int(stored.size());
+  h->nstored = nst;
   const int BP = h->bpitch;
   if (!h->lref.empty()) {
     // FP64 column-major copy on the device, mapped to L^-1 B L^-T there.
-    std::vector<double> cm(size_t(P->nnzb) * RR);
-    for (int b = 0; b < P->nnzb; ++b)
+    std::vector<double> cm(size_t(nst) * RR);
+    for (int b = 0; b < nst; ++b)
       for (int r = 0; r < R; ++r)
-        for (int c = 0; c < R; ++c) cm[size_t(b) * RR + size_t(c) * R + r] = P->blocks[size_t(b) * RR + size_t(r) * R + c];
+        for (int c = 0; c < R; ++c) cm[size_t(b) * RR + size_t(c) * R + r] = P->blocks[size_t(stored[b]) * RR + size_t(r) * R + c];
     double* d_tmp = nullptr;
     const size_t esz = h->prec == TSP_PREC_FP64 ? 8 : (h->prec == TSP_PREC_FP32 ? 4 : 2);
     if ((rc = upload(h, &d_tmp, cm.data(), cm.size()))) return create_error_from(h, rc);
     std::vector<double>().swap(cm);
     unsigned char* dblk = nullptr;
-    if ((rc = dalloc(h, &dblk, size_t(P->nnzb) * R * BP * esz))) return create_error_from(h, rc);
+    if ((rc = dalloc(h, &dblk, size_t(nst) * R * BP * esz))) return create_error_from(h, rc);
     h->d_blocks = dblk;
-    TSP_CUDA(h, cudaMemsetAsync(h->d_blocks, 0, size_t(P->nnzb) * R * BP * esz, h->stream));
-    if (h->prec == TSP_PREC_BF16 && (rc = dalloc(h, &h->d_bscale, size_t(P->nnzb)))) return create_error_from(h, rc);
+    TSP_CUDA(h, cudaMemsetAsync(h->d_blocks, 0, size_t(nst) * R * BP * esz, h->stream));
+    if (h->prec == TSP_PREC_BF16 && (rc = dalloc(h, &h->d_bscale, size_t(nst)))) return create_error_from(h, rc);
     rc = fold_blocks(h, d_tmp, R);
     dfree(h, d_tmp);
     if (rc) return create_error_from(h, rc);
@@ -1373,10 +1472,10 @@ int tsp_create_from_blocks(const tsp_block_problem* P, tsp_handle** out) {
     return TSP_OK;
   }
   const size_t esz = h->prec == TSP_PREC_FP64 ? 8 : (h->prec == TSP_PREC_FP32 ? 4 : 2);
-  std::vector<unsigned char> host(size_t(P->nnzb) * R * BP * esz, 0);
-  std::vector<float> scales(h->prec == TSP_PREC_BF16 ? size_t(P->nnzb) : 0);
-  for (int b = 0; b < P->nnzb; ++b) {
-    const double* src = P->blocks + size_t(b) * RR;
+  std::vector<unsigned char> host(size_t(nst) * R * BP * esz, 0);
+  std::vector<float> scales(h->prec == TSP_PREC_BF16 ? size_t(nst) : 0);
+  for (int b = 0; b < nst; ++b) {
+    const double* src = P->blocks + size_t(stored[b]) * RR;
     float sc = 1.0f;
     if (h->prec == TSP_PREC_BF16) {
       float m = 0.0f;
@@ -1915,23 +2014,26 @@ int tsp_export_operator(tsp_handle* h, int32_t* row_ptr, int32_t* col, double* b
     const size_t RR = size_t(h->R) * h->R;
     const int BP = h->bpitch;
     const size_t esz = h->prec == TSP_PREC_FP64 ? 8 : (h->prec == TSP_PREC_FP32 ? 4 : 2);
-    std::vector<unsigned char> raw(size_t(h->nnzb) * h->R * BP * esz);
+    std::vector<unsigned char> raw(size_t(h->nstored) * h->R * BP * esz);
     std::vector<float> sc;
     TSP_CUDA(h, copy_sync(raw.data(), h->d_blocks, raw.size(), cudaMemcpyDeviceToHost, h->stream));
     if (h->prec == TSP_PREC_BF16) {
       sc.resize(size_t(h->nnzb));
       TSP_CUDA(h, copy_sync(sc.data(), h->d_bscale, sc.size() * 4, cudaMemcpyDeviceToHost, h->stream));
     }
-    for (long long b = 0; b < h->nnzb; ++b)
+    for (long long b = 0; b < h->nnzb; ++b) {
+      const size_t at = h->bref.empty() ? size_t(b) : size_t(h->bref[b] >> 1);
+      const bool tr = !h->bref.empty() && (h->bref[b] & 1);
       for (int c = 0; c < h->R; ++c)
         for (int r = 0; r < h->R; ++r) {
-          const size_t i = size_t(b) * h->R * BP + size_t(c) * BP + r;
+          const size_t i = at * h->R * BP + size_t(tr ? r : c) * BP + (tr ? c : r);
           double v;
           if (h->prec == TSP_PREC_FP64) v = reinterpret_cast<double*>(raw.data())[i];
           else if (h->prec == TSP_PREC_FP32) v = reinterpret_cast<float*>(raw.data())[i];
           else v = double(__bfloat162float(reinterpret_cast<__nv_bfloat16*>(raw.data())[i])) * sc[b];
           blocks[size_t(b) * RR + size_t(r) * h->R + c] = v;
         }
+    }
     if (!h->lref.empty()) {
       // Stored: L^-1 B L^-T; exported: B = L (L^-1 B L^-T) L^T, applied to
       // the Np-segments of every row (right factor) and column (left factor).

@@ -419,6 +419,70 @@ void bsr_pattern(int32_t ne, const int32_t* neigh, std::vector<int32_t>* row_ptr
   }
 }
 
+int32_t symmetric_refs(int32_t ne, const int32_t* nedge, const std::vector<int32_t>& row_ptr,
+                       const std::vector<int32_t>& col, const std::vector<int8_t>& bface, std::vector<int32_t>* ref) {
+  ref->assign(col.size(), -1);
+  int32_t n = 0;
+  for (int32_t e = 0; e < ne; ++e)
+    for (int32_t b = row_ptr[e]; b < row_ptr[e + 1]; ++b)
+      if (col[b] >= e) (*ref)[b] = n++ << 1;
+  for (int32_t e = 0; e < ne; ++e)
+    for (int32_t b = row_ptr[e]; b < row_ptr[e + 1]; ++b) {
+      const int32_t f = col[b];
+      if (f >= e) continue;
+      // The neighbour's entry across the same face.
+      const int lp = nedge[3 * size_t(e) + bface[b]];
+      for (int32_t t = row_ptr[f]; t < row_ptr[f + 1]; ++t)
+        if (bface[t] == lp && col[t] == e) (*ref)[b] = (*ref)[t] | 1;
+      if ((*ref)[b] < 0) {  // a face that its neighbour pairs otherwise: every block on its own
+        for (size_t t = 0; t < col.size(); ++t) (*ref)[t] = int32_t(t) << 1;
+        return int32_t(col.size());
+      }
+    }
+  return n;
+}
+
+bool symmetric_refs_of_blocks(int32_t ne, int R, const int32_t* row_ptr, const int32_t* col, const double* blocks,
+                              std::vector<int32_t>* ref, int32_t* nstored) {
+  const size_t RR = size_t(R) * R;
+  const int32_t nnzb = row_ptr[ne];
+  ref->assign(nnzb, -1);
+  int32_t n = 0;
+  bool sym = true;
+  for (int32_t e = 0; e < ne && sym; ++e)
+    for (int32_t b = row_ptr[e]; b < row_ptr[e + 1] && sym; ++b) {
+      const int32_t f = col[b];
+      if (f == e) {
+        sym = b == row_ptr[e];  // one diagonal entry, the first of the row
+        (*ref)[b] = n++ << 1;
+        continue;
+      }
+      int32_t mirror = -1, same = 0, mirrors = 0;
+      for (int32_t t = row_ptr[f]; t < row_ptr[f + 1]; ++t)
+        if (col[t] == e) {
+          mirror = t;
+          ++mirrors;
+        }
+      for (int32_t t = row_ptr[e]; t < row_ptr[e + 1]; ++t) same += col[t] == f;
+      if (mirrors != 1 || same != 1) {
+        sym = false;
+      } else if (f > e) {
+        const double *A = blocks + size_t(b) * RR, *B = blocks + size_t(mirror) * RR;
+        for (int r = 0; r < R && sym; ++r)
+          for (int c = 0; c < R && sym; ++c) sym = A[size_t(r) * R + c] == B[size_t(c) * R + r];
+        (*ref)[b] = n++ << 1;
+      } else {
+        (*ref)[b] = (*ref)[mirror] | 1;
+      }
+    }
+  if (!sym) {
+    n = nnzb;
+    for (int32_t b = 0; b < nnzb; ++b) (*ref)[b] = b << 1;
+  }
+  *nstored = n;
+  return sym;
+}
+
 namespace {
 
 // Padded bounding box of element e. The pad covers every point the

@@ -100,6 +100,20 @@ bool build_neighbours(int32_t ne, const int32_t* tri, int32_t* neigh, int32_t* n
 void bsr_pattern(int32_t ne, const int32_t* neigh, std::vector<int32_t>* row_ptr, std::vector<int32_t>* col,
                  std::vector<int8_t>* bface);
 
+// Symmetric storage of the pattern's blocks: the diagonal blocks and, of the
+// two blocks of each interior face, the one of the lower-numbered row, in row
+// order. ref[b] = stored block of pattern entry b << 1 | transposed; returns
+// the number of stored blocks. Where the neighbour tables are not mutual (an
+// edge of more than two triangles) every block is stored, ref[b] = b << 1.
+int32_t symmetric_refs(int32_t ne, const int32_t* nedge, const std::vector<int32_t>& row_ptr,
+                       const std::vector<int32_t>& col, const std::vector<int8_t>& bface, std::vector<int32_t>* ref);
+
+// The same for a foreign pattern with values: false (and full storage, ref[b]
+// = b << 1) unless every off-diagonal entry has exactly one mirror entry whose
+// block [R][R] is its exact transpose.
+bool symmetric_refs_of_blocks(int32_t ne, int R, const int32_t* row_ptr, const int32_t* col, const double* blocks,
+                              std::vector<int32_t>* ref, int32_t* nstored);
+
 // PointWiseEntity::M_add (Receivers_imp.hpp:34-51): the lowest-id element
 // passing Triangle::intriangle (Geometry.cpp:112-118), reference coordinates
 // by invmap (Geometry.cpp:199-202) and basis values. Returns -1 if none.

@@ -85,6 +85,10 @@ struct StepParams {
   // kernel that writes a NaN or infinite u^{k+1}.
   int* nonfinite;
   long long nnzb;             // blocks of the pattern (the checked build's row bounds)
+  // Single-shot ring kernel: block references of every row (RowRefs) and the
+  // number of stored blocks.
+  const void* rows;
+  int nphys;
 };
 
 // Gather indices of the step kernels -- row extents, neighbour ids, source
@@ -1889,6 +1893,10 @@ struct AssembleParams {
   const double* Wx;          // [9][Np][Np]
   const double* Ds;          // [6][Np][Np]
   const double* Dx;          // [18][Np][Np]
+  // Symmetric storage (null: every block of the pattern is stored in its
+  // order): stored block of each pattern entry << 1 | transposed. Transposed
+  // entries are the mirror images of stored ones and are not written.
+  const int* ref;
   int prec;                  // 0 fp64, 1 fp32, 2 bf16+scale
   int pitch;                 // column pitch of a stored block (>= 2Np; padding pre-zeroed)
   void* out;                 // blocks, column-major per block
@@ -1995,6 +2003,8 @@ __global__ void __launch_bounds__(256) k_assemble(const AssembleParams p) {
   const int RR = R * R;
   for (int q = 0; q < nb; ++q) {
     const int b = rb + q, c = col_at(p, b), face = p.bface[b];
+    const int ref = p.ref ? p.ref[b] : b << 1;
+    if (ref & 1) continue;
     float inv_sc = 1.0f;
     if (p.prec == 2) {
       float amax = 0.0f;
@@ -2020,7 +2030,7 @@ __global__ void __launch_bounds__(256) k_assemble(const AssembleParams p) {
     for (int i = t; i < RR; i += blockDim.x) {
       const int cc = i / R, r = i - cc * R;  // column-major storage: (r, cc) at cc*pitch + r
       const double v = block_entry(p, e, c, face, r, cc, alpha, betas, cmn, betan[q]);
-      const size_t o = size_t(b) * R * p.pitch + size_t(cc) * p.pitch + r;
+      const size_t o = size_t(ref >> 1) * R * p.pitch + size_t(cc) * p.pitch + r;
       if (p.prec == 0) reinterpret_cast<double*>(p.out)[o] = v;
       else if (p.prec == 1) reinterpret_cast<float*>(p.out)[o] = float(v);
       else reinterpret_cast<__nv_bfloat16*>(p.out)[o] = __float2bfloat16_rn(float(v) * inv_sc);
