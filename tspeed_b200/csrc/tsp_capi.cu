@@ -24,6 +24,7 @@
 #include "tsp_dmma.cuh"
 #include "tsp_simt32.cuh"
 #include "tsp_rowring.cuh"
+#include "tsp_matfree.cuh"
 
 namespace {
 
@@ -63,8 +64,10 @@ struct tsp_handle {
   void* d_blocks = nullptr;
   float* d_bscale = nullptr;
   double* d_minv = nullptr;
-  // matrix-free operator: packed reference tables and per-element data
+  // matrix-free operator: reference tables, per-element data, and the edge
+  // values of each state level (like d_U, d_D[i] belongs to d_U[i])
   tsp::MatFreeParams mf = {};
+  double* d_D[2] = {nullptr, nullptr};
   // multi-mesh group (set by tsp_batch_create; null for ordinary handles)
   double* d_dt_elem = nullptr;
   int* d_src_of = nullptr;
@@ -671,10 +674,35 @@ int launch_d64u(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   return TSP_OK;
 }
 
+// Edge values of x into d_D[to].
+template <int N>
+int launch_matfree_traces(tsp_handle* h, const double* x, int to, cudaStream_t st) {
+  typedef tsp::MFCfg<N> CF;
+  const size_t smem = size_t(CF::TRC + CF::WARPS * CF::WS) * sizeof(double);
+  static unsigned long long configured = 0;
+  const unsigned long long bit = 1ull << (h->device & 63);
+  if (!(configured & bit)) {
+    cudaError_t e = cudaFuncSetAttribute(tsp::k_matfree_traces<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("matrix-free traces smem: ") + cudaGetErrorString(e));
+    configured |= bit;
+  }
+  tsp::MatFreeParams q = h->mf;
+  q.din = nullptr;
+  q.dout = h->d_D[to];
+  const unsigned grid = unsigned(std::min<long long>((h->ne + 7) / 8, (long long)CF::CTAS * h->num_sms));
+  tsp::k_matfree_traces<N><<<grid, CF::WARPS * 32, smem, st>>>(x, h->ne, q);
+  return TSP_OK;
+}
+
+// A step reads the edge values of its level and writes those of the new one.
+// kModeFirst computes its level's first. A single product (kModeApply,
+// kModePower) computes its vector's into the buffer that the next step will
+// write: the current level's stay valid.
 template <int N>
 int launch_matfree_N(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   typedef tsp::MFCfg<N> CF;
   const size_t smem = CF::smem_bytes();
+  static_assert(CF::smem_bytes() <= 227 * 1024, "matrix-free kernel shared memory");
   static unsigned long long configured = 0;
   const unsigned long long bit = 1ull << (h->device & 63);
   if (!(configured & bit)) {
@@ -682,12 +710,27 @@ int launch_matfree_N(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("matrix-free kernel smem: ") + cudaGetErrorString(e));
     configured |= bit;
   }
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tsp::k_step_matfree<N>, CF::WARPS * 32, smem);
-  if (per_sm < 1) per_sm = 1;
-  const long long want = (h->ne + CF::WARPS - 1) / CF::WARPS;
-  const unsigned grid = unsigned(std::min<long long>(want, (long long)per_sm * h->num_sms));
-  tsp::k_step_matfree<N><<<grid, CF::WARPS * 32, smem, st>>>(p, h->mf);
+  tsp::MatFreeParams q = h->mf;
+  const bool stepping = p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst;
+  const int from = stepping ? (p.x == h->d_U[0] ? 0 : 1) : 1 - h->cur;
+  if (p.mode != tsp::kModeStep) {
+    int rc = launch_matfree_traces<N>(h, p.x, from, st);
+    if (rc) return rc;
+  }
+  q.din = h->d_D[from];
+  q.dout = stepping ? h->d_D[1 - from] : nullptr;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(unsigned(std::min<long long>((h->ne + 7) / 8, (long long)CF::CTAS * h->num_sms)));
+  lc.blockDim = dim3(CF::WARPS * 32);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&lc, tsp::k_step_matfree<N>, p, q);
+  if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("matrix-free kernel: ") + cudaGetErrorString(e));
   return TSP_OK;
 }
 
@@ -703,6 +746,52 @@ int launch_matfree(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
     case 8: return launch_matfree_N<8>(h, p, st);
     default: return fail(h, TSP_ERR_UNSUPPORTED, "matrix-free kernel: N must be in 1..8");
   }
+}
+
+int refresh_matfree(tsp_handle* h, int i) {
+  switch (h->N) {
+    case 1: return launch_matfree_traces<1>(h, h->d_U[i], i, h->stream);
+    case 2: return launch_matfree_traces<2>(h, h->d_U[i], i, h->stream);
+    case 3: return launch_matfree_traces<3>(h, h->d_U[i], i, h->stream);
+    case 4: return launch_matfree_traces<4>(h, h->d_U[i], i, h->stream);
+    case 5: return launch_matfree_traces<5>(h, h->d_U[i], i, h->stream);
+    case 6: return launch_matfree_traces<6>(h, h->d_U[i], i, h->stream);
+    case 7: return launch_matfree_traces<7>(h, h->d_U[i], i, h->stream);
+    default: return launch_matfree_traces<8>(h, h->d_U[i], i, h->stream);
+  }
+}
+
+// Packed tables of MFCfg<N>, in fragment order.
+std::vector<double> matfree_tables(int N, const tsp::RefTables& T) {
+  const int Np = T.Np, Q = T.Q, RQ = 3 * Q;
+  const int KS = (Np + 3) / 4, MT = (Np + 7) / 8, TT = (RQ + 7) / 8, KL = (3 * RQ + 3) / 4;
+  const size_t P2 = size_t(Np) * Np;
+  auto edge = [&](int part, int r, int j) {  // part 0: basis value, 1 + a: derivative a, at edge point r
+    const int l = r / Q, kq = r % Q;
+    return part == 0 ? T.Be[(size_t(l) * Q + kq) * Np + j] : T.Ge[((size_t(l) * 2 + (part - 1)) * Q + kq) * Np + j];
+  };
+  std::vector<double> pk;
+  for (int ab = 0; ab < 4; ++ab)
+    for (int t = 0; t < MT; ++t)
+      for (int ks = 0; ks < KS; ++ks)
+        for (int lane = 0; lane < 32; ++lane) {
+          const int i = 8 * t + lane / 4, j = 4 * ks + lane % 4;
+          pk.push_back(i < Np && j < Np ? T.K[ab * P2 + size_t(i) * Np + j] : 0.0);
+        }
+  for (int t = 0; t < MT; ++t)
+    for (int ks = 0; ks < KL; ++ks)
+      for (int lane = 0; lane < 32; ++lane) {
+        const int i = 8 * t + lane / 4, kk = 4 * ks + lane % 4;
+        pk.push_back(i < Np && kk < 3 * RQ ? T.w1[(kk % RQ) % Q] * edge(kk / RQ, kk % RQ, i) : 0.0);
+      }
+  for (int part = 0; part < 3; ++part)
+    for (int t = 0; t < TT; ++t)
+      for (int ks = 0; ks < KS; ++ks)
+        for (int lane = 0; lane < 32; ++lane) {
+          const int r = 8 * t + lane / 4, j = 4 * ks + lane % 4;
+          pk.push_back(r < RQ && j < Np ? edge(part, r, j) : 0.0);
+        }
+  return pk;
 }
 
 template <int R, int ST, int TR>
@@ -978,8 +1067,10 @@ int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, d
   }
 }
 
-// Rebuilds the FP32 shadow of state level i from its FP64 values.
+// Rebuilds what the step kernels keep beside state level i (the FP32 shadow,
+// the matrix-free edge values) from its FP64 values.
 int refresh_shadow(tsp_handle* h, int i) {
+  if (h->op_kind == TSP_OP_MATRIX_FREE) return refresh_matfree(h, i);
   if (!h->shadow) return TSP_OK;
   const int ntile = (h->S + 63) / 64;
   tsp::k_make_shadow<<<1184, 256, 0, h->stream>>>(h->d_U[i], h->d_X32[i], h->ne, h->S, h->R, ntile);
@@ -1260,40 +1351,31 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
     return create_error_from(h, rc);
   h->bpitch = block_pitch(h->R, h->S);
   if (h->op_kind == TSP_OP_MATRIX_FREE) {
-    // Packed tables in the kernel's shared-memory layout: KT[ab][j][i],
-    // TRT[l][j][r], TR[l][r][i] (r < Q: basis, Q <= r < 3Q: gradient a = r/Q-1), w1.
-    const int Np = h->Np, Q = T.Q, Q3 = 3 * Q;
-    const size_t P2 = size_t(Np) * Np;
-    std::vector<double> pk(4 * P2 + 2 * size_t(3) * Np * Q3 + Q);
-    double* KT = pk.data();
-    double* TRT = KT + 4 * P2;
-    double* TR = TRT + size_t(3) * Np * Q3;
-    double* W1 = TR + size_t(3) * Q3 * Np;
-    for (int ab = 0; ab < 4; ++ab)
-      for (int i = 0; i < Np; ++i)
-        for (int j = 0; j < Np; ++j) KT[(size_t(ab) * Np + j) * Np + i] = T.K[ab * P2 + size_t(i) * Np + j];
-    for (int l = 0; l < 3; ++l)
-      for (int r = 0; r < Q3; ++r)
-        for (int j = 0; j < Np; ++j) {
-          const int kq = r % Q, part = r / Q;
-          const double v = part == 0 ? T.Be[(size_t(l) * Q + kq) * Np + j]
-                                     : T.Ge[((size_t(l) * 2 + (part - 1)) * Q + kq) * Np + j];
-          TRT[(size_t(l) * Np + j) * Q3 + r] = v;
-          TR[(size_t(l) * Q3 + r) * Np + j] = v;
-        }
-    for (int kq = 0; kq < Q; ++kq) W1[kq] = T.w1[kq];
-    double* d_tab = nullptr;
-    if ((rc = upload(h, &d_tab, pk.data(), pk.size()))) return create_error_from(h, rc);
+    const std::vector<double> pk = matfree_tables(P->N, T);
+    double *d_tab = nullptr, *d_alpha = nullptr, *d_face = nullptr;
+    int* d_nbr = nullptr;
+    const size_t nd = size_t(h->ne) * 3 * T.Q * 4;
+    if ((rc = upload(h, &d_tab, pk.data(), pk.size())) || (rc = dalloc(h, &d_alpha, size_t(h->ne) * 10)) ||
+        (rc = dalloc(h, &d_face, size_t(h->ne) * 36)) || (rc = dalloc(h, &d_nbr, size_t(h->ne) * 3)) ||
+        (rc = dalloc(h, &h->d_D[0], nd)) || (rc = dalloc(h, &h->d_D[1], nd)))
+      return create_error_from(h, rc);
+    for (int i = 0; i < 2; ++i) TSP_CUDA(h, cudaMemsetAsync(h->d_D[i], 0, nd * sizeof(double), h->stream));
+    tsp::k_matfree_geometry<<<(h->ne + 127) / 128, 128, 0, h->stream>>>(h->ne, d_invJ, d_detJ, d_lam, d_mu, d_elen,
+                                                                        d_enrm, d_neigh, d_nedge,
+                                                                        P->penalty * h->N * h->N, d_alpha, d_face, d_nbr);
+    cudaError_t ge = cudaGetLastError();
+    if (ge == cudaSuccess) ge = cudaStreamSynchronize(h->stream);
+    if (ge != cudaSuccess) {
+      fail(h, TSP_ERR_CUDA, std::string("matrix-free geometry: ") + cudaGetErrorString(ge));
+      return create_error_from(h, TSP_ERR_CUDA);
+    }
     h->mf.tables = d_tab;
-    h->mf.invJ = d_invJ;
-    h->mf.detJ = d_detJ;
-    h->mf.lam = d_lam;
-    h->mf.mu = d_mu;
-    h->mf.elen = d_elen;
-    h->mf.enrm = d_enrm;
-    h->mf.neigh = d_neigh;
-    h->mf.nedge = d_nedge;
-    h->mf.pen_n2 = P->penalty * h->N * h->N;
+    h->mf.alpha = d_alpha;
+    h->mf.face = d_face;
+    h->mf.nbr = d_nbr;
+    for (void* q : {(void*)d_neigh, (void*)d_nedge, (void*)d_invJ, (void*)d_detJ, (void*)d_elen, (void*)d_enrm,
+                    (void*)d_lam, (void*)d_mu})
+      dfree(h, q);
     for (void* q : {(void*)d_bface, (void*)d_K, (void*)d_Ws, (void*)d_Wx, (void*)d_Ds, (void*)d_Dx}) dfree(h, q);
     if ((rc = finish_create(h))) return create_error_from(h, rc);
     *out = h;

@@ -27,7 +27,8 @@
 // Programmatic dependent launch: the blocks and row references never change,
 // so a step's warps fill their rings before they wait for the previous step
 // (griddepcontrol.wait); everything that a step writes or reads of the state
-// comes after that wait.
+// comes after that wait, by ordinary loads: the read-only path does not hold
+// for data that changes while the grid waits.
 //
 // Products: a chunk holds NC columns of the stored block (column-major, pitch
 // 2Np). Untransposed, lanes own row pairs (G groups of lanes share the columns
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     const double2* src = reinterpret_cast<const double2*>(p.x + size_t(unsigned(c < 0 ? 0 : c)) * R) + lane;
 #pragma unroll
     for (int s = 0; s < PPL; ++s)
-      if (lane + 32 * s < NPAIR) xv[s] = __ldg(src + 32 * s);
+      if (lane + 32 * s < NPAIR) xv[s] = src[32 * s];
   };
   // What the epilogue of a row needs, requested a row ahead by the warp whose turn it is.
   double2 uk[PPL], up[PPL];
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     for (int s = 0; s < PPL; ++s) {
       uk[s] = up[s] = make_double2(0.0, 0.0);
       if (lane + 32 * s < NPAIR) {
-        uk[s] = __ldg(src + 32 * s);
+        uk[s] = src[32 * s];
         if (stepping && p.uprev != nullptr) up[s] = prv[32 * s];
       }
     }
