@@ -1,0 +1,144 @@
+"""Kernels on symmetric block storage and the matrix-free tiles at the sizes
+where they can go wrong (GPU), against the oracle's products and recurrence.
+
+Tolerances: FP64 paths differ from the oracle in summation order only,
+1e-13 of the result's norm for a product and 1e-12 over a few steps. FP32
+operators hold each entry to 2^-24 of itself and, with one shot, sum at most
+4 * 90 FP32 products per row: 360 * 2^-24 = 2.2e-5 bounds the relative error
+of rows without cancellation; 1e-4 covers the few steps taken here."""
+import numpy as np
+import pytest
+
+import tsp_oracle as O
+from helpers import rel
+from tspeed_b200 import capi
+from tspeed_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def random_operator(ne, N, seed, symmetric):
+    """A block-CSR operator on a random graph of degree 0..3 (rows of 1..4
+    blocks, diagonal first); symmetric: block (f, e) is the transpose of
+    (e, f), else every block is its own."""
+    rng = np.random.default_rng(seed)
+    R = (N + 1) * (N + 2)
+    nb = [[] for _ in range(ne)]
+    for e in range(ne):
+        for f in rng.permutation(ne)[:6]:
+            if f != e and f not in nb[e] and len(nb[e]) < 3 and len(nb[f]) < 3:
+                nb[e].append(int(f))
+                nb[int(f)].append(e)
+    row_ptr, col, blocks = [0], [], []
+    at = {}
+    for e in range(ne):
+        for f in [e] + nb[e]:
+            B = rng.uniform(0.5, 1.0, size=(R, R)) / R
+            if symmetric and f == e:
+                B = 0.5 * (B + B.T)
+            if symmetric and f < e:
+                B = blocks[at[(f, e)]].T
+            at[(e, f)] = len(col)
+            col.append(f)
+            blocks.append(np.ascontiguousarray(B))
+        row_ptr.append(len(col))
+    minv = rng.uniform(0.5, 2.0, size=ne)
+    return np.array(row_ptr, np.int32), np.array(col, np.int32), np.array(blocks), minv
+
+
+# One row, rows without neighbours, fewer rows than teams, and more rows than
+# one round of teams; every degree that the ring kernel takes and one below.
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("N,ne", [(2, 40), (3, 1), (3, 700), (4, 61), (5, 2), (5, 601), (6, 37), (7, 9), (8, 33)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_single_shot_blocks(N, ne, symmetric, precision):
+    row_ptr, col, blocks, minv = random_operator(ne, N, 7 * N + ne, symmetric)
+    Np = (N + 1) * (N + 2) // 2
+    rng = np.random.default_rng(ne)
+    u0, v0 = rng.standard_normal((2, 2 * ne * Np))
+    phi = rng.standard_normal((3, Np))
+    rcv = [0, ne // 2, ne - 1]
+    F = rng.standard_normal((4, 2))
+    with capi.Simulation.from_blocks(row_ptr, col, blocks, minv, [ne - 1], phi[:1], rcv, phi, precision=precision) as s:
+        y = s.apply(u0)
+        assert rel(s.export_operator()[2], blocks) < (1e-15 if precision == "fp64" else 1e-7)
+        s.set_dt(0.01)
+        s.set_force_table(0, F)
+        s.set_initial(0, u0, v0)
+        s.first_step()
+        s.step()
+        s.run(2)
+        u, seis = s.u(), s.seismograms(0, 4)[0]
+    tol = (1e-13, 1e-12) if precision == "fp64" else (1e-4, 1e-4)
+    assert rel(y, O.apply_B(row_ptr, col, blocks, u0, ne, Np)) < tol[0]
+    ur, sr, _ = O.leapfrog(row_ptr, col, blocks, minv, ne, Np, 0.01, 4, ne - 1, phi[0], F, rcv, phi, u0, v0)
+    assert rel(u, ur) < tol[1]
+    assert rel(seis, sr) < tol[1]
+
+
+# Shot counts at the edges of the 8-, 16-, 24- and 32-shot tiles and of one, two and three tiles.
+@pytest.mark.parametrize("N,S", [(3, 2), (3, 8), (3, 33), (4, 9), (4, 65), (5, 16), (5, 17), (5, 24), (6, 25), (6, 48),
+                                 (7, 32), (7, 70), (8, 3), (8, 24)])
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_few_shots(N, S, symmetric, precision, monkeypatch):
+    monkeypatch.delenv("TSP_BATCHED_VARIANT", raising=False)
+    ne = 11
+    row_ptr, col, blocks, minv = random_operator(ne, N, N + S, symmetric)
+    Np = (N + 1) * (N + 2) // 2
+    rng = np.random.default_rng(S)
+    u0 = rng.standard_normal((S, 2 * ne * Np))
+    sphi = rng.standard_normal((S, Np))
+    se = rng.integers(0, ne, size=S)
+    rphi = rng.standard_normal((2, Np))
+    rcv = [4, 4]
+    F = rng.standard_normal((S, 3, 2))
+    with capi.Simulation.from_blocks(row_ptr, col, blocks, minv, se, sphi, rcv, rphi, precision=precision) as s:
+        y = s.apply(u0[0])
+        s.set_dt(0.01)
+        for k in range(S):
+            s.set_force_table(k, F[k])
+            s.set_initial(k, u0[k])
+        s.first_step()
+        s.run(2)
+        u, seis = s.u_all(), s.seismograms(0, 3)
+    tol = (1e-13, 1e-12) if precision == "fp64" else (1e-4, 1e-4)
+    assert rel(y, O.apply_B(row_ptr, col, blocks, u0[0], ne, Np)) < tol[0]
+    for k in range(S):
+        ur, sr, _ = O.leapfrog(row_ptr, col, blocks, minv, ne, Np, 0.01, 3, int(se[k]), sphi[k], F[k], rcv, rphi, u0[k])
+        assert rel(u[k], ur) < tol[1]
+        assert rel(seis[k], sr) < tol[1]
+
+
+# Element counts around the tile of eight, and more tiles than one round of warps.
+@pytest.mark.parametrize("N", range(1, 9))
+@pytest.mark.parametrize("nx,ny", [(1, 1), (3, 1), (2, 2), (3, 3), (5, 5), (60, 57)])
+def test_matrix_free_tiles(N, nx, ny):
+    if nx == 60 and N > 4:
+        nx, ny = 31, 29
+    m = W.jittered_rect(nx, ny, 100.0 * nx, 100.0 * ny, seed=N)
+    rng = np.random.default_rng(N)
+    vp = 2500 + 1500 * rng.random(m.ne)
+    lam, mu, rho = W.lame(vp, vp / 1.8, 2000 + 500 * rng.random(m.ne))
+    out = {}
+    x = rng.standard_normal(m.ne * (N + 1) * (N + 2))
+    for op in ("explicit", "matrix_free"):
+        with capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(40.0, 30.0)], [(61.0, 33.0), (20.0, 55.0)],
+                                    penalty=10.0, op=op) as s:
+            y = s.apply(x)
+            lmax = s.estimate_lmax(20)
+            s.set_dt(0.3 * 2 / np.sqrt(lmax) if op == "explicit" else out["explicit"][4])
+            dt = 0.3 * 2 / np.sqrt(lmax)
+            s.set_ricker(0, 20.0, 0.05, -1e9, 1, 20)
+            s.set_initial(0, 1e-3 * x)
+            s.enable_energy(True)
+            s.first_step()
+            s.run(9)
+            s.apply(x)  # a product between steps leaves the state's edge values alone
+            s.run(6)
+            out[op] = (y, s.u(), s.seismograms(0, 16), s.energy(1, 15), dt, lmax)
+    a, b = out["matrix_free"], out["explicit"]
+    assert rel(a[0], b[0]) < 1e-13
+    assert abs(a[5] - b[5]) < 1e-12 * b[5]
+    for i in (1, 2, 3):
+        assert rel(a[i], b[i]) < 1e-11

@@ -25,6 +25,7 @@
 #include "tsp_simt32.cuh"
 #include "tsp_rowring.cuh"
 #include "tsp_matfree.cuh"
+#include "tsp_rowshots.cuh"
 
 namespace {
 
@@ -373,6 +374,10 @@ int autotune(tsp_handle* h) {
   NvtxRange nvtx_("autotune");
   const bool fx_ok = h->fx;
   const bool fp64_batched = h->S > 1 && h->prec == TSP_PREC_FP64 && h->op_kind == TSP_OP_EXPLICIT;
+  if (h->S > 1 && h->d_rows) {  // few shots: the DMMA step on symmetric storage
+    h->kernel_variant = h->prec == TSP_PREC_FP64 ? 5 : 14;
+    return TSP_OK;
+  }
   if (fp64_batched) {
     if (h->kernel_variant >= 0) {
       const int v = h->kernel_variant;
@@ -499,9 +504,33 @@ int upload_rows(tsp_handle* h, const int* row_ptr, const int* col) {
 // 2Np = 20 65 / 50, 30 70 / 97). BF16 blocks are not multiples of the 16 bytes
 // of a bulk copy.
 constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 30); }
+// Handles of a few shots use the same storage with shot tiles of 8 to 32
+// (k_step_rowshots), unless TSP_BATCHED_VARIANT asks for a batched kernel.
+// Most shots for which that is the faster one (0: any number), from 4,900
+// triangles, us per step, few-shot kernel / best batched kernel:
+//   FP64  2Np = 20: S = 48 57 / 63, 64 73 / 65; 30: 24 52 / 128, 64 116 / 143;
+//         42: 8 41 / 187, 48 182 / 197, 64 248 / 206; 56: 64 336 / 414;
+//         72: 8 110 / 300, 64 630 / 674; 90: 8 150 / 380, 24 372 / 389, 32 478 / 394
+//   FP32  20: 32 36 / 50, 64 73 / 58; 30: 8 23 / 69, 32 67 / 77, 48 98 / 84;
+//         42: 24 99 / 118, 32 131 / 121; 56: 48 247 / 252, 64 337 / 258;
+//         72: 8 79 / 608, 64 502 / 686; 90: 8 107 / 796, 64 823 / 962
+constexpr bool rowshots_size(int R) { return R >= 20; }
+int rowshots_max(int R, bool fp64) {
+  switch (R) {
+    case 20: return fp64 ? 48 : 32;
+    case 30: return fp64 ? 0 : 32;
+    case 42: return fp64 ? 48 : 24;
+    case 56: return fp64 ? 0 : 48;
+    case 90: return fp64 ? 24 : 0;
+    default: return 0;
+  }
+}
 bool uses_rowring(const tsp_handle* h) {
-  return h->S == 1 && h->op_kind == TSP_OP_EXPLICIT && h->prec != TSP_PREC_BF16 &&
-         rowring_size(h->R, h->prec == TSP_PREC_FP64);
+  if (h->op_kind != TSP_OP_EXPLICIT || h->prec == TSP_PREC_BF16) return false;
+  const bool fp64 = h->prec == TSP_PREC_FP64;
+  if (h->S == 1) return rowring_size(h->R, fp64);
+  const int most = rowshots_max(h->R, fp64);
+  return rowshots_size(h->R) && h->kernel_variant < 0 && (most == 0 || h->S <= most);
 }
 
 int finish_create(tsp_handle* h) {
@@ -513,7 +542,7 @@ int finish_create(tsp_handle* h) {
   }
   // The FP32 batched kernel (FP32 blocks, several shots, 2Np <= 72) keeps an
   // FP32 transposed shadow of each state level.
-  h->shadow = (h->S > 1 && h->prec == TSP_PREC_FP32 && h->R <= 72);
+  h->shadow = (h->S > 1 && h->prec == TSP_PREC_FP32 && h->R <= 72 && !h->d_rows);
   if (h->shadow) {
     const int ntile = (h->S + 63) / 64;
     const size_t nsh = size_t(h->ne) * ntile * h->R * 64;
@@ -914,13 +943,59 @@ int launch_rowring(tsp_handle* h, const tsp::StepParams& p0, cudaStream_t st) {
   return TSP_OK;
 }
 
+// Step of a few shots on symmetric storage: persistent, one CTA per SM.
+template <int R, int ST, typename BT>
+int launch_rowshots(tsp_handle* h, const tsp::StepParams& p0, cudaStream_t st) {
+  typedef tsp::RowShotsCfg<R, ST, BT> CF;
+  constexpr size_t smem = CF::smem_bytes();
+  static_assert(smem <= 227 * 1024, "few-shot kernel shared memory");
+  static unsigned long long configured = 0;
+  const unsigned long long bit = 1ull << (h->device & 63);
+  auto kern = tsp::k_step_rowshots<R, ST, BT>;
+  if (!(configured & bit)) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("few-shot kernel smem: ") + cudaGetErrorString(e));
+    configured |= bit;
+  }
+  tsp::StepParams p = p0;
+  p.rows = h->d_rows;
+  p.nphys = int(h->nstored);
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(unsigned(std::min<long long>((long long)p.ne * ((p.S + ST - 1) / ST), h->num_sms)));
+  lc.blockDim = dim3(CF::NT);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = &at;
+  lc.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&lc, kern, p, h->d_err);
+  if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("few-shot kernel: ") + cudaGetErrorString(e));
+  return TSP_OK;
+}
+
+// The fewest tiles of at most 32 shots, as even as steps of 8 allow.
+template <int R, typename BT>
+int launch_rowshots_of(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
+  const int ntile = (h->S + 31) / 32, st8 = (h->S + 8 * ntile - 1) / (8 * ntile);
+  switch (st8) {
+    case 1: return launch_rowshots<R, 8, BT>(h, p, st);
+    case 2: return launch_rowshots<R, 16, BT>(h, p, st);
+    case 3: return launch_rowshots<R, 24, BT>(h, p, st);
+    default: return launch_rowshots<R, 32, BT>(h, p, st);
+  }
+}
+
 template <int R>
 int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   if (h->d_rows) {
-    if constexpr (rowring_size(R, true))
-      if (h->prec == TSP_PREC_FP64) return launch_rowring<R, double>(h, p, st);
-    if constexpr (rowring_size(R, false))
-      if (h->prec == TSP_PREC_FP32) return launch_rowring<R, float>(h, p, st);
+    if constexpr (rowshots_size(R)) {
+      const bool fp64 = h->prec == TSP_PREC_FP64;
+      if (h->S > 1 && (p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst))
+        return fp64 ? launch_rowshots_of<R, double>(h, p, st) : launch_rowshots_of<R, float>(h, p, st);
+      return fp64 ? launch_rowring<R, double>(h, p, st) : launch_rowring<R, float>(h, p, st);
+    }
   }
   if constexpr (R <= 56) {
     if (h->fx && (p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst)) return launch_fx<R>(h, p, st);
@@ -1349,7 +1424,7 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
       (rc = upload(h, &d_Ws, T.Ws.data(), T.Ws.size())) || (rc = upload(h, &d_Wx, T.Wx.data(), T.Wx.size())) ||
       (rc = upload(h, &d_Ds, T.Ds.data(), T.Ds.size())) || (rc = upload(h, &d_Dx, T.Dx.data(), T.Dx.size())))
     return create_error_from(h, rc);
-  h->bpitch = block_pitch(h->R, h->S);
+  h->bpitch = h->bref.empty() ? block_pitch(h->R, h->S) : h->R;
   if (h->op_kind == TSP_OP_MATRIX_FREE) {
     const std::vector<double> pk = matfree_tables(P->N, T);
     double *d_tab = nullptr, *d_alpha = nullptr, *d_face = nullptr;
@@ -1514,7 +1589,7 @@ int tsp_create_from_blocks(const tsp_block_problem* P, tsp_handle** out) {
   // Transpose every block to column-major and convert to the storage type.
   const int R = h->R;
   const size_t RR = size_t(R) * R;
-  h->bpitch = block_pitch(R, h->S);
+  h->bpitch = uses_rowring(h) ? R : block_pitch(R, h->S);
   // The stored blocks, as entries of the pattern.
   std::vector<int> stored;
   if (uses_rowring(h)) {
