@@ -508,12 +508,12 @@ constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 30); }
 // (k_step_rowshots), unless TSP_BATCHED_VARIANT asks for a batched kernel.
 // Most shots for which that is the faster one (0: any number), from 4,900
 // triangles, us per step, few-shot kernel / best batched kernel:
-//   FP64  2Np = 20: S = 48 57 / 63, 64 73 / 65; 30: 24 52 / 128, 64 116 / 143;
-//         42: 8 41 / 187, 48 182 / 197, 64 248 / 206; 56: 64 336 / 414;
-//         72: 8 110 / 300, 64 630 / 674; 90: 8 150 / 380, 24 372 / 389, 32 478 / 394
-//   FP32  20: 32 36 / 50, 64 73 / 58; 30: 8 23 / 69, 32 67 / 77, 48 98 / 84;
-//         42: 24 99 / 118, 32 131 / 121; 56: 48 247 / 252, 64 337 / 258;
-//         72: 8 79 / 608, 64 502 / 686; 90: 8 107 / 796, 64 823 / 962
+//   FP64  2Np = 20: S = 48 57 / 63, 64 73 / 65; 30: 24 49 / 128, 64 116 / 143;
+//         42: 8 37 / 187, 48 172 / 197, 64 230 / 206; 56: 64 336 / 414;
+//         72: 8 96 / 300, 64 630 / 674; 90: 8 140 / 380, 48 575 / 753, 64 791 / 755
+//   FP32  20: 32 36 / 50, 64 73 / 58; 30: 8 19 / 69, 32 67 / 77, 48 98 / 84;
+//         42: 24 91 / 118, 32 130 / 121; 56: 48 247 / 252, 64 337 / 258;
+//         72: 8 72 / 608, 64 502 / 686; 90: 8 104 / 796, 64 823 / 962
 constexpr bool rowshots_size(int R) { return R >= 20; }
 int rowshots_max(int R, bool fp64) {
   switch (R) {
@@ -521,7 +521,7 @@ int rowshots_max(int R, bool fp64) {
     case 30: return fp64 ? 0 : 32;
     case 42: return fp64 ? 48 : 24;
     case 56: return fp64 ? 0 : 48;
-    case 90: return fp64 ? 24 : 0;
+    case 90: return fp64 ? 48 : 0;
     default: return 0;
   }
 }

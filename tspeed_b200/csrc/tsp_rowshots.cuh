@@ -38,14 +38,40 @@
 
 namespace tsp {
 
+// Row tiles per warp and groups of a CTA. Measured on 4,900 triangles, us per
+// step (tiles, groups): FP64 2Np = 20, 8 shots (1, 6) 17.0, (3, 12) 14.1; 42,
+// 24 shots (1, 3) 95, (2, 4) 86; 72, 8 shots (1, 2) 108, (3, 2) 96; 90, 24
+// shots (2, 1) 369, (1, 1) 288. FP32 2Np = 30, 8 shots (1, 4) 21.3, (4, 12)
+// 18.8; 42, 24 shots (1, 3) 99, (2, 5) 91; 72, 8 shots (1, 2) 75.5, (3, 4)
+// 71.8; 90, 24 shots (1, 1) 292, (2, 2) 285. More row tiles per warp read the
+// state's fragments fewer times and leave more warps to other rows, until
+// the accumulators and the requested state levels spill.
+constexpr int rowshots_tiles(int R, int ST, bool fp64) {
+  switch (R) {
+    case 20: return ST == 8 ? 3 : 1;
+    case 30: return ST == 8 && !fp64 ? 4 : ST <= 24 && fp64 ? 2 : 1;
+    case 42: return 2;
+    case 72: return ST == 8 ? 3 : 1;
+    case 90: return fp64 ? 1 : 2;
+    default: return 1;
+  }
+}
+constexpr int rowshots_groups(int R, int ST, bool fp64) {
+  switch (R) {
+    case 20: return ST == 8 ? 12 : 6;
+    case 30: return ST == 8 && !fp64 ? 12 : ST <= 24 && fp64 ? 6 : 4;
+    case 42: return fp64 || ST == 32 ? 4 : 5;
+    case 72: return ST == 8 && !fp64 ? 4 : 2;
+    default: return 2;
+  }
+}
+
 template <int R, int ST, typename BT>
 struct RowShotsCfg {
   static constexpr int KS = (R + 3) / 4;
   static constexpr int NTL = (R + 7) / 8;
   static constexpr int MT = ST / 8;
-  // Row tiles per warp and groups: enough independent accumulators and enough
-  // rows in flight to cover the ring's latency.
-  static constexpr int NTW = R == 90 ? 2 : 1;
+  static constexpr int NTW = rowshots_tiles(R, ST, sizeof(BT) == 8);
   static constexpr int WN = (NTL + NTW - 1) / NTW;
   static constexpr int BB = R * R * int(sizeof(BT));  // bytes: the block
   static constexpr int XB = ST * R * 8;               // the state tile
@@ -54,7 +80,9 @@ struct RowShotsCfg {
   static_assert(8 * NTL - R <= ST, "fragment rows past the block stay inside the stage");
   static_assert((8 * NTL - R) * R * int(sizeof(BT)) <= XB, "fragment rows past the block stay inside the stage");
   static constexpr int total() { return int((226 * 1024) / (STAGE + 16)); }
-  static constexpr int NG = R <= 20 ? 6 : R <= 30 ? 4 : R <= 42 ? 3 : total() >= 4 ? 2 : 1;
+  // One group where two rings of two stages do not fit.
+  static constexpr int NG0 = rowshots_groups(R, ST, sizeof(BT) == 8);
+  static constexpr int NG = total() / NG0 >= 2 ? NG0 : 1;
   static constexpr int NSG = total() / NG > 6 ? 6 : total() / NG;
   static_assert(NSG >= 2, "two stages per group must fit");
   static constexpr int NST = NG * NSG;
