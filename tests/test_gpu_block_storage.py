@@ -142,3 +142,27 @@ def test_matrix_free_tiles(N, nx, ny):
     assert abs(a[5] - b[5]) < 1e-12 * b[5]
     for i in (1, 2, 3):
         assert rel(a[i], b[i]) < 1e-11
+
+
+def test_large_read_back_matches_small_ones():
+    """Copies of several megabytes pass through the pinned pieces, small ones
+    do not: wrapped seismogram rings with rows above one 8 MiB piece, many
+    rows per piece, and a whole wavefield of several shots."""
+    m = W.jittered_rect(40, 40, 4000.0, 4000.0, seed=3)
+    lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+    shots = [(1000.0 + 37 * k, 3900.0) for k in range(6)]
+    rcv = [(4000.0 * (r + 0.37) / 257, 3933.0) for r in range(257)]
+    with capi.Simulation.create(m.xy, m.tri, 3, lam, mu, rho, shots, rcv, penalty=10.0) as s:
+        s.set_dt(1e-4)
+        for k in range(6):
+            s.set_ricker(k, 20.0, 0.01, -1e9, 1, 3000)
+        s.set_seismogram_capacity(2100)
+        s.first_step()
+        s.run(2999)  # the ring wraps inside [900, 3000)
+        for k0, n in ((900, 2100), (1700, 300)):  # rows of 8.6 MB and of 1.2 MB
+            big = s.seismograms(k0, n)
+            small = np.concatenate([s.seismograms(k0 + i, min(15, n - i)) for i in range(0, n, 15)], axis=1)
+            assert np.array_equal(big, small)
+        u = s.u_all()
+        for k in range(6):
+            assert np.array_equal(u[k], s.u(k))

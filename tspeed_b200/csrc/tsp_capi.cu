@@ -18,6 +18,7 @@
 
 #include "../../include/tspeed_b200.h"
 #include "tsp_host.h"
+#include "tsp_readback.h"
 #include "tsp_kernels.cuh"
 #include "tsp_tcgen05.cuh"
 #include "tsp_tcfx.cuh"
@@ -1246,10 +1247,31 @@ int reset_nonfinite(tsp_handle* h) {
   return TSP_OK;
 }
 
+// Shots [shot, shot + n) of ne elements of a device state buffer in the
+// reference's layout, transposed on the device. TSP_ERR_NOMEM where the
+// transposed copy does not fit.
+int get_shots(tsp_handle* h, const double* dsrc, int ne, int shot, int n, double* out) {
+  const size_t nref = size_t(2) * ne * h->Np;
+  double* tmp = nullptr;
+  int rc = dalloc(h, &tmp, nref * n);
+  if (rc) return rc;
+  tsp::k_state_to_ref<<<1184, 256, 0, h->stream>>>(dsrc, ne, h->S, h->Np, shot, n, tmp, h->d_lref_inv);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = tsp::read_back(out, nref * n * sizeof(double), tmp, nref * n * sizeof(double), nref * n * sizeof(double), 1,
+                       h->stream);
+  dfree(h, tmp);
+  if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("state read-back: ") + cudaGetErrorString(e));
+  return TSP_OK;
+}
+
 // One shot's slice of a device state buffer (ne runs of R doubles with a
 // stride of S*R) to/from a reference-layout host vector (NULL: zeros).
-int get_shot(tsp_handle* h, const double* dsrc, int shot, double* out) {
-  const int ne = h->ne, R = h->R;
+int get_shot(tsp_handle* h, const double* dsrc, int ne, int shot, double* out) {
+  const int R = h->R;
+  const int rc = get_shots(h, dsrc, ne, shot, 1, out);
+  if (rc != TSP_ERR_NOMEM) return rc;
+  // No room on the device: reorder on the host.
   std::vector<double> slice(size_t(ne) * R);
   TSP_CUDA(h, cudaMemcpy2DAsync(slice.data(), size_t(R) * sizeof(double), dsrc + size_t(shot) * R,
                                 size_t(h->S) * R * sizeof(double), size_t(R) * sizeof(double), ne,
@@ -1682,6 +1704,7 @@ int tsp_release_cached_memory(int32_t device) {
     std::lock_guard<std::mutex> lk(g_pool_mutex);
     pool = g_pools[device];
   }
+  tsp::Staging::get().release();
   if (!pool) return TSP_OK;
   int prev = 0;
   cudaGetDevice(&prev);
@@ -1931,7 +1954,7 @@ int tsp_get_u(tsp_handle* h, int32_t shot, double* out) {
   if (shot < 0 || shot >= h->S) return fail(h, TSP_ERR_ARG, "shot out of range");
   int rc;
   if ((rc = begin(h))) return rc;
-  if ((rc = get_shot(h, h->d_U[h->cur], shot, out))) return rc;
+  if ((rc = get_shot(h, h->d_U[h->cur], h->ne, shot, out))) return rc;
   return check_device_error(h);
 }
 
@@ -1944,20 +1967,8 @@ int tsp_get_u_all(tsp_handle* h, double* out) {
   // of shots at a time, and each chunk is copied back in one transfer.
   const size_t nref = size_t(2) * h->ne * h->Np;
   const int chunk = int(std::max<size_t>(1, std::min<size_t>(size_t(h->S), (size_t(256) << 20) / (nref * 8))));
-  double* tmp = nullptr;
-  if ((rc = dalloc(h, &tmp, nref * chunk))) return rc;
-  for (int s0 = 0; s0 < h->S && rc == TSP_OK; s0 += chunk) {
-    const int ns = std::min(chunk, h->S - s0);
-    tsp::k_state_to_ref<<<1184, 256, 0, h->stream>>>(h->d_U[h->cur], h->ne, h->S, h->Np, s0, ns, tmp,
-                                                     h->d_lref_inv);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(out + size_t(s0) * nref, tmp, nref * ns * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) rc = fail(h, TSP_ERR_CUDA, std::string("state read-back: ") + cudaGetErrorString(e));
-  }
-  dfree(h, tmp);
-  if (rc) return rc;
+  for (int s0 = 0; s0 < h->S; s0 += chunk)
+    if ((rc = get_shots(h, h->d_U[h->cur], h->ne, s0, std::min(chunk, h->S - s0), out + size_t(s0) * nref))) return rc;
   return check_device_error(h);
 }
 
@@ -1981,16 +1992,15 @@ int tsp_get_seismograms(tsp_handle* h, int64_t k0, int64_t nk, double* out) {
   int rc;
   if ((rc = begin(h))) return rc;
   const size_t per = size_t(h->nrcv) * 2;
-  for (int s = 0; s < h->S; ++s)
-    for (int64_t k = 0; k < nk;) {
-      // Contiguous run inside the ring buffer.
-      const long long slot = (k0 + k) % h->seis_cap;
-      const long long run = std::min<long long>(nk - k, h->seis_cap - slot);
-      TSP_CUDA(h, cudaMemcpyAsync(out + (size_t(s) * nk + k) * per, h->d_seis + (size_t(s) * h->seis_cap + slot) * per,
-                                  size_t(run) * per * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-      k += run;
-    }
-  TSP_CUDA(h, cudaStreamSynchronize(h->stream));
+  for (int64_t k = 0; k < nk;) {
+    // A run inside the ring buffer, the same one for every shot.
+    const long long slot = (k0 + k) % h->seis_cap;
+    const long long run = std::min<long long>(nk - k, h->seis_cap - slot);
+    TSP_CUDA(h, tsp::read_back(out + size_t(k) * per, size_t(nk) * per * sizeof(double), h->d_seis + size_t(slot) * per,
+                               size_t(h->seis_cap) * per * sizeof(double), size_t(run) * per * sizeof(double), h->S,
+                               h->stream));
+    k += run;
+  }
 #ifdef TSP_CHECKED
   return check_device_error(h);  // the samples are void after an index failure
 #else
@@ -3042,15 +3052,8 @@ int tsp_batch_get_u(tsp_batch* b, int32_t mesh, double* out) {
   tsp_handle* h = b->groups[b->mesh_group[mesh]];
   cudaSetDevice(b->device);
   cudaStreamSynchronize(b->stream);
-  const int Np = h->Np, R = h->R, ne = b->mesh_ne[mesh];
-  std::vector<double> v(size_t(ne) * R);
-  if (copy_sync(v.data(), h->d_U[h->cur] + size_t(b->mesh_first[mesh]) * R, v.size() * sizeof(double),
-                cudaMemcpyDeviceToHost, h->stream) != cudaSuccess)
-    return bfail(b, TSP_ERR_CUDA, "state read-back failed");
-  for (int e = 0; e < ne; ++e)
-    for (int c = 0; c < 2; ++c)
-      std::memcpy(out + size_t(c) * ne * Np + size_t(e) * Np, &v[size_t(e) * R + size_t(c) * Np], Np * sizeof(double));
-  return TSP_OK;
+  const int rc = get_shot(h, h->d_U[h->cur] + size_t(b->mesh_first[mesh]) * h->R, b->mesh_ne[mesh], 0, out);
+  return rc ? bfail(b, rc, h->err) : TSP_OK;
 }
 
 int tsp_batch_get_seismograms(tsp_batch* b, int32_t mesh, int64_t k0, int64_t nk, double* out) {
@@ -3061,11 +3064,20 @@ int tsp_batch_get_seismograms(tsp_batch* b, int32_t mesh, int64_t k0, int64_t nk
   const int nr = b->mesh_nrcv[mesh], r0 = b->mesh_rcv0[mesh];
   if (nr == 0 || nk == 0) return TSP_OK;
   if (nk > h->seis_cap) return bfail(b, TSP_ERR_ARG, "range longer than the seismogram capacity");
-  std::vector<double> all(size_t(nk) * h->nrcv * 2);
-  int rc = tsp_get_seismograms(h, k0, nk, all.data());
+  // The mesh's receivers are consecutive in every step's samples of the group.
+  const size_t row = size_t(nr) * 2 * sizeof(double), pitch = size_t(h->nrcv) * 2 * sizeof(double);
+  for (int64_t k = 0; k < nk;) {
+    const long long slot = (k0 + k) % h->seis_cap;
+    const long long run = std::min<long long>(nk - k, h->seis_cap - slot);
+    const cudaError_t e = tsp::read_back(out + size_t(k) * nr * 2, row, h->d_seis + (size_t(slot) * h->nrcv + r0) * 2,
+                                         pitch, row, size_t(run), h->stream);
+    if (e != cudaSuccess) return bfail(b, TSP_ERR_CUDA, std::string("seismogram read-back: ") + cudaGetErrorString(e));
+    k += run;
+  }
+#ifdef TSP_CHECKED
+  const int rc = check_device_error(h);
   if (rc) return bfail(b, rc, h->err);
-  for (int64_t k = 0; k < nk; ++k)
-    std::memcpy(out + size_t(k) * nr * 2, &all[(size_t(k) * h->nrcv + r0) * 2], size_t(nr) * 2 * sizeof(double));
+#endif
   return TSP_OK;
 }
 
