@@ -109,6 +109,7 @@ struct tsp_handle {
   int* d_rcv_ptr = nullptr;
   int* d_rcv_id = nullptr;
   double* d_rcv_phi = nullptr;
+  double* d_rcv_phi_q = nullptr;  // in the order of d_rcv_id
   double* d_seis = nullptr;
   long long seis_cap = 0;
   double* d_energy = nullptr;
@@ -282,6 +283,10 @@ int build_receiver_csr(tsp_handle* h) {
   std::vector<double> rphi(h->rcv_phi);
   if (!h->lref_inv.empty()) map_vectors(h->lref_inv, false, h->Np, rphi.data(), h->nrcv);
   if ((rc = upload(h, &h->d_rcv_phi, rphi.data(), rphi.size()))) return rc;
+  std::vector<double> qphi(rphi.size());
+  for (int q = 0; q < h->nrcv; ++q)
+    std::copy(&rphi[size_t(ids[q]) * h->Np], &rphi[size_t(ids[q]) * h->Np] + h->Np, &qphi[size_t(q) * h->Np]);
+  if ((rc = upload(h, &h->d_rcv_phi_q, qphi.data(), qphi.size()))) return rc;
   return TSP_OK;
 }
 
@@ -343,7 +348,7 @@ int fx_dispatch(tsp_handle* h, bool setup, int i) {
 }
 
 int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, double* out, int rel,
-                double xscale, cudaStream_t st);
+                double xscale, cudaStream_t st, double* acc = nullptr, const double* acc_prev = nullptr);
 int check_device_error(tsp_handle* h);
 
 // Autotuner of the batched step kernels: each applicable kernel variant
@@ -913,14 +918,14 @@ int launch_ksplit(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
 
 // Single-shot ring kernel: persistent, one team of four warps per CTA, launched with programmatic stream serialization so that a step's rings fill
 // while the previous step ends.
-template <int R, typename BT>
+template <int R, typename BT, bool ORD = false>
 int launch_rowring(tsp_handle* h, const tsp::StepParams& p0, cudaStream_t st) {
   typedef tsp::RowRingCfg<R, BT> CF;
   constexpr size_t smem = CF::smem_bytes();
   static_assert(CF::CTAS >= 1 && CF::CTAS * (smem + 1024) <= 228 * 1024, "row ring kernel shared memory");
   static unsigned long long configured = 0;
   const unsigned long long bit = 1ull << (h->device & 63);
-  auto kern = tsp::k_step_rowring<R, BT>;
+  auto kern = tsp::k_step_rowring<R, BT, ORD>;
   if (!(configured & bit)) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("row ring kernel smem: ") + cudaGetErrorString(e));
@@ -993,9 +998,12 @@ int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   if (h->d_rows) {
     if constexpr (rowshots_size(R)) {
       const bool fp64 = h->prec == TSP_PREC_FP64;
-      if (h->S > 1 && (p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst))
+      const bool stepping = p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst;
+      if (h->S > 1 && stepping)
         return fp64 ? launch_rowshots_of<R, double>(h, p, st) : launch_rowshots_of<R, float>(h, p, st);
-      return fp64 ? launch_rowring<R, double>(h, p, st) : launch_rowring<R, float>(h, p, st);
+      return fp64       ? launch_rowring<R, double>(h, p, st)
+             : stepping ? launch_rowring<R, float>(h, p, st)
+                        : launch_rowring<R, float, true>(h, p, st);
     }
   }
   if constexpr (R <= 56) {
@@ -1073,7 +1081,7 @@ int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
 }
 
 int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, double* out, int rel,
-                double xscale, cudaStream_t st) {
+                double xscale, cudaStream_t st, double* acc, const double* acc_prev) {
   tsp::StepParams p;
   std::memset(&p, 0, sizeof(p));
   p.ne = h->ne;
@@ -1100,6 +1108,7 @@ int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, d
   p.rcv_ptr = (sample && h->nrcv > 0) ? h->d_rcv_ptr : nullptr;
   p.rcv_id = h->d_rcv_id;
   p.rcv_phi = h->d_rcv_phi;
+  p.rcv_phi_q = h->d_rcv_phi_q;
   p.seis = h->d_seis;
   p.nrcv = h->nrcv;
   p.seis_cap = h->seis_cap;
@@ -1107,7 +1116,8 @@ int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, d
   p.nonfinite = sample ? h->d_err + 1 : nullptr;
   p.nnzb = h->nnzb;
   p.energy_cap = h->energy_cap;
-  p.acc = h->d_acc;
+  p.acc = acc ? acc : h->d_acc;
+  p.acc_prev = acc_prev;
   p.x32_in = nullptr;
   p.x32_out = nullptr;
   if (h->shadow) {
@@ -1323,6 +1333,83 @@ int make_handle(int device, tsp_handle** out) {
     return fail(nullptr, TSP_ERR_CUDA, std::string("stream creation: ") + cudaGetErrorString(e));
   }
   *out = h;
+  return TSP_OK;
+}
+
+// The first n numbers of the power iterations' start vector (a deterministic
+// vector with all modes excited: the xorshift64 sequence), generated on the
+// device. The step of the sequence is linear over GF(2), so the state 512
+// numbers on is a fixed 64 x 64 bit matrix times the state: the host walks the
+// chunks' first states, the device fills the chunks.
+int start_vector(tsp_handle* h, double* d_x, size_t n) {
+  typedef unsigned long long u64;
+  auto next = [](u64 st) {
+    st ^= st << 13;
+    st ^= st >> 7;
+    st ^= st << 17;
+    return st;
+  };
+  u64 M[64], T[64];  // columns: images of the unit vectors
+  for (int i = 0; i < 64; ++i) M[i] = next(1ull << i);
+  auto apply = [](const u64* A, u64 v) {
+    u64 r = 0;
+    for (int i = 0; v; ++i, v >>= 1)
+      if (v & 1) r ^= A[i];
+    return r;
+  };
+  static_assert(tsp::kXorChunk == 512, "nine squarings");
+  for (int q = 0; q < 9; ++q) {
+    for (int i = 0; i < 64; ++i) T[i] = apply(M, M[i]);
+    std::copy(T, T + 64, M);
+  }
+  const size_t chunks = (n + tsp::kXorChunk - 1) / tsp::kXorChunk;
+  std::vector<u64> seed(chunks);
+  u64 st = 0x9E3779B97F4A7C15ull;
+  for (size_t c = 0; c < chunks; ++c) {
+    seed[c] = st;
+    st = apply(M, st);
+  }
+  u64* d_seed = nullptr;
+  int rc = upload(h, &d_seed, seed.data(), seed.size());
+  if (rc) return rc;
+  tsp::k_xorshift_fill<<<unsigned((chunks + 63) / 64), 64, 0, h->stream>>>(d_seed, d_x, n);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);  // `seed` ends here
+  dfree(h, d_seed);
+  if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("start vector: ") + cudaGetErrorString(e));
+  return TSP_OK;
+}
+
+// `iters` power iterations of M^-1 B on one vector per mesh (one mesh for an
+// ordinary handle); acc: the last iteration's sums, three per mesh. Every
+// iteration adds its sums to a slot of its own and scales its vector by the
+// slot before, so the iterations follow one another without the host.
+int power_iterate(tsp_handle* h, int nmesh, int iters, double* acc) {
+  const size_t n1 = size_t(h->ne) * h->R;  // one vector, layout [e][R]
+  const int half = std::min(iters, 256);
+  const size_t per = 3 * size_t(nmesh);
+  double *da = nullptr, *db = nullptr, *ring = nullptr;
+  int rc;
+  if (!(rc = dalloc(h, &da, n1)) && !(rc = dalloc(h, &db, n1)) && !(rc = dalloc(h, &ring, 2 * half * per)))
+    rc = start_vector(h, da, n1);
+  auto slot = [&](int it) { return ring + size_t(it / half % 2 * half + it % half) * per; };
+  cudaError_t e = cudaSuccess;
+  for (int it = 0; it < iters && !rc && e == cudaSuccess; ++it) {
+    // A half's slots are cleared when it is entered: the slot before lies in the other half.
+    if (it % half == 0) e = cudaMemsetAsync(slot(it), 0, half * per * sizeof(double), h->stream);
+    if (e == cudaSuccess)
+      rc = launch_step(h, tsp::kModePower, da, nullptr, db, 0, 1.0, h->stream, slot(it), it ? slot(it - 1) : nullptr);
+    if (!rc && e == cudaSuccess) e = cudaGetLastError();
+    std::swap(da, db);
+  }
+  if (!rc && e == cudaSuccess)
+    e = cudaMemcpyAsync(acc, slot(iters - 1), per * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
+  const cudaError_t s = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) e = s;
+  for (double* q : {da, db, ring})
+    if (q) dfree(h, q);
+  if (rc) return rc;
+  if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("power iteration: ") + cudaGetErrorString(e));
   return TSP_OK;
 }
 
@@ -2137,33 +2224,9 @@ int tsp_estimate_lmax(tsp_handle* h, int32_t iters, double* lmax) {
   if (!h || !lmax || iters < 1) return TSP_ERR_ARG;
   int rc;
   if ((rc = begin(h))) return rc;
-  const size_t nstate = size_t(h->ne) * h->R;  // one vector, layout [e][R]
-  double *da = nullptr, *db = nullptr;
-  if ((rc = dalloc(h, &da, nstate)) || (rc = dalloc(h, &db, nstate))) return rc;
-  // Deterministic start vector with all modes excited.
-  std::vector<double> x0(nstate);
-  uint64_t st = 0x9E3779B97F4A7C15ull;
-  for (size_t i = 0; i < nstate; ++i) {
-    st ^= st << 13;
-    st ^= st >> 7;
-    st ^= st << 17;
-    x0[i] = double(st >> 11) * (1.0 / 9007199254740992.0) - 0.5;
-  }
-  TSP_CUDA(h, copy_sync(da, x0.data(), nstate * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  double scale = 1.0, lam = 0.0;
   double acc[3];
-  for (int it = 0; it < iters; ++it) {
-    TSP_CUDA(h, cudaMemsetAsync(h->d_acc, 0, 3 * sizeof(double), h->stream));
-    if ((rc = launch_step(h, tsp::kModePower, da, nullptr, db, 0, scale, h->stream))) return rc;
-    TSP_CUDA(h, cudaMemcpyAsync(acc, h->d_acc, sizeof(acc), cudaMemcpyDeviceToHost, h->stream));
-    TSP_CUDA(h, cudaStreamSynchronize(h->stream));
-    lam = acc[0] / acc[1];  // Rayleigh quotient x^T B x / x^T M x
-    scale = acc[2] > 0 ? 1.0 / std::sqrt(acc[2]) : 1.0;
-    std::swap(da, db);
-  }
-  *lmax = lam;
-  dfree(h, da);
-  dfree(h, db);
+  if ((rc = power_iterate(h, 1, iters, acc))) return rc;
+  *lmax = acc[0] / acc[1];  // Rayleigh quotient x^T B x / x^T M x
   return TSP_OK;
 }
 
@@ -2835,9 +2898,11 @@ int tsp_batch_create(const tsp_problem* meshes, int32_t nmesh, tsp_batch** out) 
     dfree(h, h->d_rcv_ptr);
     dfree(h, h->d_rcv_id);
     dfree(h, h->d_rcv_phi);
+    dfree(h, h->d_rcv_phi_q);
     h->d_rcv_ptr = nullptr;
     h->d_rcv_id = nullptr;
     h->d_rcv_phi = nullptr;
+    h->d_rcv_phi_q = nullptr;
     std::vector<double> ones(ms.size(), 1.0);
     if ((rc = upload(h, &h->d_src_phi, src_phi.data(), src_phi.size())) ||
         (rc = upload(h, &h->d_src_of, src_of.data(), src_of.size())) ||
@@ -2877,40 +2942,10 @@ int tsp_batch_estimate_lmax(tsp_batch* b, int32_t iters, double* lmax) {
   for (size_t g = 0; g < b->groups.size(); ++g) {
     tsp_handle* h = b->groups[g];
     const int nm = h->nmesh;
-    const size_t n1 = size_t(h->ne) * h->R;
-    double *da = nullptr, *db = nullptr;
-    int rc;
-    if ((rc = dalloc(h, &da, n1)) || (rc = dalloc(h, &db, n1))) return bfail(b, rc, h->err);
-    std::vector<double> x0(n1);
-    uint64_t st = 0x9E3779B97F4A7C15ull;
-    for (size_t i = 0; i < n1; ++i) {
-      st ^= st << 13;
-      st ^= st >> 7;
-      st ^= st << 17;
-      x0[i] = double(st >> 11) * (1.0 / 9007199254740992.0) - 0.5;
-    }
-    if (copy_sync(da, x0.data(), n1 * sizeof(double), cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
-      return bfail(b, TSP_ERR_CUDA, "upload of the start vector failed");
-    std::vector<double> scale(nm, 1.0), acc(3 * size_t(nm)), lam(nm, 0.0);
-    for (int it = 0; it < iters; ++it) {
-      if (cudaMemcpyAsync(h->d_xscale_mesh, scale.data(), nm * sizeof(double), cudaMemcpyHostToDevice, h->stream) !=
-              cudaSuccess ||
-          cudaMemsetAsync(h->d_acc, 0, 3 * size_t(nm) * sizeof(double), h->stream) != cudaSuccess)
-        return bfail(b, TSP_ERR_CUDA, "power iteration setup failed");
-      if ((rc = launch_step(h, tsp::kModePower, da, nullptr, db, 0, 1.0, h->stream))) return bfail(b, rc, h->err);
-      if (cudaMemcpyAsync(acc.data(), h->d_acc, acc.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream) !=
-              cudaSuccess ||
-          cudaStreamSynchronize(h->stream) != cudaSuccess)
-        return bfail(b, TSP_ERR_CUDA, std::string("power iteration: ") + cudaGetErrorString(cudaGetLastError()));
-      for (int q = 0; q < nm; ++q) {
-        lam[q] = acc[3 * q] / acc[3 * q + 1];
-        scale[q] = acc[3 * q + 2] > 0 ? 1.0 / std::sqrt(acc[3 * q + 2]) : 1.0;
-      }
-      std::swap(da, db);
-    }
-    for (int q = 0; q < nm; ++q) lmax[b->group_meshes[g][q]] = lam[q];
-    dfree(h, da);
-    dfree(h, db);
+    std::vector<double> acc(3 * size_t(nm));
+    const int rc = power_iterate(h, nm, iters, acc.data());
+    if (rc) return bfail(b, rc, h->err);
+    for (int q = 0; q < nm; ++q) lmax[b->group_meshes[g][q]] = acc[3 * q] / acc[3 * q + 1];
   }
   return TSP_OK;
 }

@@ -43,6 +43,9 @@ struct StepParams {
   double* out;                // u^{k+1}; may alias uprev (same thread reads then writes)
   double dt;
   double xscale;              // kModePower: x is used as xscale*x
+  // kModePower: sums of the iteration before (3 per mesh); x is then scaled by
+  // 1/sqrt of the third instead of xscale.
+  const double* acc_prev;
   const long long* step_base; // device step counter (k = *step_base + rel)
   int rel;
   // sources: one point source per shot
@@ -54,6 +57,7 @@ struct StepParams {
   const int* rcv_ptr;         // [ne+1] or null
   const int* rcv_id;          // [nrcv] receiver ids ordered by element
   const double* rcv_phi;      // [nrcv][Np] by receiver id
+  const double* rcv_phi_q;    // [nrcv][Np] in the order of rcv_id
   double* seis;               // [S][cap][nrcv][2]
   int nrcv;
   long long seis_cap;
@@ -142,6 +146,44 @@ __device__ __forceinline__ int rcv_ptr_at(const StepParams& p, int e) {
 // Receiver id of entry q (indexes rcv_phi and the seismogram buffer).
 __device__ __forceinline__ int rcv_id_at(const StepParams& p, int q) {
   return TSP_INDEX(p.rcv_id[q], 0, p.nrcv, kSiteRcvId);
+}
+
+// Scale of x in a power iteration, for element e.
+__device__ __forceinline__ double power_scale(const StepParams& p, int e) {
+  if (p.acc_prev != nullptr) {
+    const double s = p.acc_prev[3 * size_t(p.mesh_of != nullptr ? p.mesh_of[e] : 0) + 2];
+    return s > 0 ? 1.0 / sqrt(s) : 1.0;
+  }
+  return p.xscale_mesh ? p.xscale_mesh[p.mesh_of[e]] : p.xscale;
+}
+
+// Receivers [q0, q1) of one element sampled by a whole warp: lanes share the
+// modes, y(c, i) is mode i of component c of the new level. (One lane per
+// receiver and component walked its modes with a dependent load each: 1.4 us
+// of the 11 us step of 1,600 triangles at N = 4 with 8 receivers, 10 us of
+// 255 at 40,000 triangles, N = 5 with 128.)
+template <int NP, class Y>
+__device__ __forceinline__ void sample_receivers(const StepParams& p, int q0, int q1, long long k, int sh, int lane,
+                                                 Y y) {
+  const long long slot = k % p.seis_cap;
+  for (int q = q0; q < q1; ++q) {
+    const int rid = rcv_id_at(p, q);
+    double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < NP; i += 32)
+      if (i + lane < NP) {
+        const double ph = __ldg(p.rcv_phi_q + size_t(q) * NP + i + lane);
+        v0 = fma(ph, y(0, i + lane), v0);
+        v1 = fma(ph, y(1, i + lane), v1);
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    if (lane == 0)
+      *reinterpret_cast<double2*>(p.seis + ((size_t(sh) * p.seis_cap + slot) * p.nrcv + rid) * 2) = make_double2(v0, v1);
+  }
 }
 
 // Raises the non-finite flag when a new displacement pair holds a NaN or an
@@ -268,7 +310,7 @@ __global__ void __launch_bounds__(256) k_step_rows(const StepParams p) {
     for (int b = 0; b < nb; ++b) {
       const int c = col_at(p, rb + b);
       const double2* src = reinterpret_cast<const double2*>(p.x + (size_t(c) * S + sh) * R);
-      const double xs = (p.mode == kModePower) ? (p.xscale_mesh ? p.xscale_mesh[p.mesh_of[e]] : p.xscale) : 1.0;
+      const double xs = (p.mode == kModePower) ? power_scale(p, e) : 1.0;
       for (int q = tl; q < NPAIR; q += T) {
         double2 v = __ldg(src + q);
         if (p.mode == kModePower) { v.x *= xs; v.y *= xs; }
@@ -1514,6 +1556,22 @@ __global__ void k_state_to_ref(const double* __restrict__ u, int ne, int S, int 
     } else {
       out[o] = w[i];
     }
+  }
+}
+
+// kXorChunk states of the xorshift64 sequence from each seed on, as numbers
+// in [-0.5, 0.5): the power iterations' start vector.
+constexpr int kXorChunk = 512;
+__global__ void k_xorshift_fill(const unsigned long long* __restrict__ seed, double* __restrict__ x, size_t n) {
+  const size_t c = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (c * kXorChunk >= n) return;
+  unsigned long long st = seed[c];
+  const size_t end = n < (c + 1) * kXorChunk ? n : (c + 1) * kXorChunk;
+  for (size_t i = c * kXorChunk; i < end; ++i) {
+    st ^= st << 13;
+    st ^= st >> 7;
+    st ^= st << 17;
+    x[i] = double(st >> 11) * (1.0 / 9007199254740992.0) - 0.5;
   }
 }
 

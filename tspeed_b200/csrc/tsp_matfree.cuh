@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
         al[2 * i + 1] = v.y;
       }
       if (p.mode == kModePower) {
-        const double xsc = p.xscale_mesh ? p.xscale_mesh[p.mesh_of[eg]] : p.xscale;
+        const double xsc = power_scale(p, eg);
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
           xb[ks][0] *= xsc;
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
       mf_load_faces<N>(q, e8, ne, lane, fc);
       __syncwarp();
       double xsc = 1.0;
-      if (p.mode == kModePower) xsc = p.xscale_mesh ? p.xscale_mesh[p.mesh_of[e]] : p.xscale;
+      if (p.mode == kModePower) xsc = power_scale(p, e);
 #pragma unroll 3
       for (int r = lane >> 3; r < RQ; r += 4) {
         const int l = r >= 2 * Q ? 2 : r >= Q ? 1 : 0, kq = r - l * Q;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
       const int srow = !stepping ? -1 : p.src_of ? p.src_of[ec]
                                       : ((p.src_elem != nullptr && src_elem_at(p, 0) == ec) ? 0 : -1);
       const bool is_src = srow >= 0 && k < p.nF;
-      const double xsc = p.mode != kModePower ? 1.0 : p.xscale_mesh ? p.xscale_mesh[p.mesh_of[ec]] : p.xscale;
+      const double xsc = p.mode != kModePower ? 1.0 : power_scale(p, ec);
       double* og = p.out + size_t(ec) * R;
       double pe0 = 0.0, pe1 = 0.0, pe2 = 0.0;
 #pragma unroll
@@ -476,16 +476,10 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
       const int last = min(e8 + 8, ne);
       const int t0 = rcv_ptr_at(p, e8), t1 = rcv_ptr_at(p, last);
       if (t1 > t0) {
-        const long long slot = k % p.seis_cap;
         for (int e = e8; e < last; ++e) {
           const int r0 = rcv_ptr_at(p, e), r1 = rcv_ptr_at(p, e + 1);
-          for (int t = lane; t < 2 * (r1 - r0); t += 32) {
-            const int rid = rcv_id_at(p, r0 + t / 2), c = t & 1;
-            const double* ph = p.rcv_phi + size_t(rid) * NP;
-            double v = 0.0;
-            for (int i = 0; i < NP; ++i) v += ph[i] * rows[c * CF::ROWS * 8 + mf_at(i, e - e8)];
-            p.seis[(size_t(slot) * p.nrcv + rid) * 2 + c] = v;
-          }
+          sample_receivers<NP>(p, r0, r1, k, 0, lane,
+                               [&](int c, int i) { return rows[c * CF::ROWS * 8 + mf_at(i, e - e8)]; });
         }
       }
     }

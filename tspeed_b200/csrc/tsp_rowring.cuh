@@ -40,6 +40,8 @@
 
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "tsp_kernels.cuh"
 #include "tsp_tcfx.cuh"
 #include "tsp_tcgen05.cuh"
@@ -122,10 +124,16 @@ __device__ __forceinline__ void row_barrier(int id, bool wait) {
   else row_barrier_id<3>(wait);
 }
 
-template <int R, typename BT>
+// ORD: every row's FP32 products are summed in column order, block by block
+// (the order of k_step_rows), for single products (kModeApply, kModePower) of
+// FP32 operators: their results stay the same to FP64 rounding whichever
+// storage the handle has. The steps take the faster order.
+template <int R, typename BT, bool ORD = false>
 __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(const StepParams p, int* err_flag) {
   typedef RowRingCfg<R, BT> CF;
   typedef typename AccOf<BT>::type AT;
+  constexpr int G = ORD ? 1 : CF::G, PT = ORD ? 1 : CF::PT, JN = ORD ? CF::NPAIR : CF::JN;
+  constexpr bool ROT = CF::ROT && !ORD;
   constexpr int NP = R / 2, NPAIR = CF::NPAIR, NC = CF::NC, NCH = CF::NCH, NS = CF::NS, PPL = CF::PPL, W = CF::W;
   constexpr int DEPTH = CF::DEPTH, LAP = CF::LAP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -220,6 +228,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
       }
     }
   };
+  const double xsc_all = p.mode == kModePower && p.mesh_of == nullptr ? power_scale(p, 0) : 1.0;
   int e = blockIdx.x;
 #pragma unroll
   for (int s = 0; s < PPL; ++s) xv[s] = make_double2(0.0, 0.0);
@@ -237,7 +246,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     const int d = DEPTH > 1 ? i % DEPTH : 0;
     double xsc = 1.0;
     if (p.mode == kModePower) {
-      xsc = p.xscale_mesh ? p.xscale_mesh[p.mesh_of[e]] : p.xscale;
+      xsc = p.mesh_of != nullptr ? power_scale(p, e) : xsc_all;
 #pragma unroll
       for (int s = 0; s < PPL; ++s) {
         xv[s].x *= xsc;
@@ -291,20 +300,20 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
       AT acc[PPL][2];
 #pragma unroll
       for (int q = 0; q < PPL; ++q) acc[q][0] = acc[q][1] = AT(0);
-      const int g = CF::G > 1 ? lane / NPAIR : 0;
-      const int pl = CF::G > 1 ? lane - g * NPAIR : lane;
+      const int g = G > 1 ? lane / NPAIR : 0;
+      const int pl = G > 1 ? lane - g * NPAIR : lane;
 #pragma unroll 1
       for (int ch = 0; ch < NCH; ++ch) {
         const BT* st = land(ch) + 2 * pl;
         const AT* xc = xs + ch * NC;
-        if constexpr (CF::G > 1) {
-          constexpr int CI = (NC + CF::G - 1) / CF::G;  // columns per group
+        if constexpr (G > 1) {
+          constexpr int CI = (NC + G - 1) / G;  // columns per group
           constexpr int UN = CI % 7 == 0 ? 7 : CI % 5 == 0 ? 5 : 6;
-          if (g < CF::G) {
+          if (g < G) {
 #pragma unroll UN
             for (int ci = 0; ci < CI; ++ci) {
-              const int cc = g + ci * CF::G;
-              if (NC % CF::G == 0 || cc < NC) {
+              const int cc = g + ci * G;
+              if (NC % G == 0 || cc < NC) {
                 AT w0, w1;
                 lds_pair(st + cc * R, w0, w1);
                 acc[0][0] = fma(w0, xc[cc], acc[0][0]);
@@ -314,7 +323,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
           }
         } else {
           // Two columns per step: one load brings both x.
-          static_assert(CF::G > 1 || NC % 2 == 0, "column pairs");
+          static_assert(G > 1 || NC % 2 == 0, "column pairs");
           constexpr int UN = NC % 14 == 0 ? 7 : NC % 10 == 0 ? 5 : NC % 8 == 0 ? 4 : 3;
 #pragma unroll UN
           for (int cc = 0; cc < NC; cc += 2) {
@@ -339,10 +348,10 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
 #pragma unroll
       for (int q = 0; q < PPL; ++q) {
         double v0 = double(acc[q][0]), v1 = double(acc[q][1]);
-        if constexpr (CF::G > 1) {
+        if constexpr (G > 1) {
           double t0 = v0, t1 = v1;
 #pragma unroll
-          for (int gg = 1; gg < CF::G; ++gg) {
+          for (int gg = 1; gg < G; ++gg) {
             t0 += __shfl_sync(0xffffffffu, v0, (pl + gg * NPAIR) & 31);
             t1 += __shfl_sync(0xffffffffu, v1, (pl + gg * NPAIR) & 31);
           }
@@ -354,9 +363,9 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
       }
     } else {
       const int pt = lane / CF::LC, lc = lane - pt * CF::LC;
-      const bool work = pt < CF::PT;
-      const int jb = work ? pt * CF::JN : 0;
-      const int len = NPAIR % CF::PT == 0 ? CF::JN : (NPAIR - jb < CF::JN ? NPAIR - jb : CF::JN);
+      const bool work = pt < PT;
+      const int jb = work ? pt * JN : 0;
+      const int len = NPAIR % PT == 0 ? JN : (NPAIR - jb < JN ? NPAIR - jb : JN);
 #pragma unroll 1
       for (int ch = 0; ch < NCH; ++ch) {
         const BT* st = land(ch) + (work ? lc : 0) * R + 2 * jb;
@@ -364,11 +373,11 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
         AT s0[CF::CPL], s1[CF::CPL];
 #pragma unroll
         for (int c = 0; c < CF::CPL; ++c) s0[c] = s1[c] = AT(0);
-        int jj = CF::ROT ? lc % CF::JN : 0;
+        int jj = ROT ? lc % JN : 0;
 #pragma unroll 7
-        for (int t = 0; t < CF::JN; ++t) {
-          const int o = CF::ROT ? 2 * jj : 2 * t;
-          if (NPAIR % CF::PT == 0 || t < len) {
+        for (int t = 0; t < JN; ++t) {
+          const int o = ROT ? 2 * jj : 2 * t;
+          if (NPAIR % PT == 0 || t < len) {
             AT x0, x1;
             lds_pair(xc + o, x0, x1);
 #pragma unroll
@@ -376,17 +385,18 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
               AT w0, w1;
               lds_pair(st + c * CF::LC * R + o, w0, w1);
               s0[c] = fma(w0, x0, s0[c]);
-              s1[c] = fma(w1, x1, s1[c]);
+              if constexpr (ORD) s0[c] = fma(w1, x1, s0[c]);
+              else s1[c] = fma(w1, x1, s1[c]);
             }
           }
-          if (CF::ROT) jj = jj + 1 == CF::JN ? 0 : jj + 1;
+          if (ROT) jj = jj + 1 == JN ? 0 : jj + 1;
         }
 #pragma unroll
         for (int c = 0; c < CF::CPL; ++c) {
           const double v = double(s0[c]) + double(s1[c]);
           double tot = v;
 #pragma unroll
-          for (int q = 1; q < CF::PT; ++q) tot += __shfl_sync(0xffffffffu, v, (lc + q * CF::LC) & 31);
+          for (int q = 1; q < PT; ++q) tot += __shfl_sync(0xffffffffu, v, (lc + q * CF::LC) & 31);
           if (pt == 0) y[ch * NC + lc + c * CF::LC] = tot;
         }
         refill(ch);
@@ -416,12 +426,13 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
         const int q = lane + 32 * s;
         un2[s] = make_double2(0.0, 0.0);
         if (q >= NPAIR) continue;
-        double yy[2] = {0.0, 0.0};
+        typename std::conditional<ORD, AT, double>::type ya = 0, yb = 0;
         for (int b = 0; b < nb_e; ++b) {
           const double2 v = *reinterpret_cast<const double2*>(yr + b * R + 2 * q);
-          yy[0] += v.x;
-          yy[1] += v.y;
+          ya += decltype(ya)(v.x);
+          yb += decltype(yb)(v.y);
         }
+        const double yy[2] = {double(ya), double(yb)};
         double u[2] = {uk[s].x, uk[s].y};
         if (p.mode == kModePower) {
           u[0] *= xsc;
@@ -462,15 +473,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
           if (q < NPAIR) *reinterpret_cast<double2*>(yw + 2 * q) = un2[s];
         }
         __syncwarp();
-        const long long slot = k % p.seis_cap;
-        for (int t = lane; t < 2 * (r1 - r0); t += 32) {
-          const int rid = rcv_id_at(p, r0 + t / 2);
-          const int comp = t & 1;
-          const double* ph = p.rcv_phi + size_t(rid) * NP;
-          double v = 0.0;
-          for (int ii = 0; ii < NP; ++ii) v += ph[ii] * yw[comp * NP + ii];
-          p.seis[(size_t(slot) * p.nrcv + rid) * 2 + comp] = v;
-        }
+        sample_receivers<NP>(p, r0, r1, k, 0, lane, [&](int c, int i) { return yw[c * NP + i]; });
       }
       // ---- per-mesh power-iteration sums (multi-mesh groups) ----
       if (p.mode == kModePower && p.mesh_of != nullptr) {

@@ -347,6 +347,7 @@ __global__ void __launch_bounds__(RowShotsCfg<R, ST, BT>::NT, 1) k_step_rowshots
             const double* ph = p.rcv_phi + size_t(rid) * NP;
             const double* un = p.out + (size_t(e) * S + sh) * R + cmp * NP;
             double v = 0.0;
+#pragma unroll(NP <= 21 ? NP : 9)
             for (int ii = 0; ii < NP; ++ii) v += ph[ii] * un[ii];
             p.seis[((size_t(sh) * p.seis_cap + slot) * p.nrcv + rid) * 2 + cmp] = v;
           }
