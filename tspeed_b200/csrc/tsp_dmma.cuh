@@ -323,6 +323,7 @@ __global__ void __launch_bounds__(d64w_nt<R, NSG, NG, WM, WN, NU, RA>(), MINB)
                 uk[mt][q] = *reinterpret_cast<const double2*>(Xs + ((wm * MTW + mt) * 8 + gs) * R + r0);
             }
         }
+        fx_reads_done();
         __syncwarp();
         if (lane == 0) fx_mbar_arrive(smem_u32(&gempty[s]));
       }

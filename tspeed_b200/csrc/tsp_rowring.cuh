@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     const unsigned char* next = block_at(ref[DEPTH]);
     const bool more = col[DEPTH] >= 0;
     auto refill = [&](int ch) {
+      fx_reads_done();
       __syncwarp();
       if (lane == 0 && !dead) {
         if constexpr (NS < NCH) {

@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(RowShotsCfg<R, ST, BT>::NT, 1) k_step_rowshots
 #pragma unroll
             for (int q = 0; q < NTW; ++q) dmma_m8n8k4(acc[mt][q][0], acc[mt][q][1], a[mt], bb[q]);
         }
+        fx_reads_done();
         __syncwarp();
         if (lane == 0) fx_mbar_arrive(smem_u32(&gempty[s]));
       }

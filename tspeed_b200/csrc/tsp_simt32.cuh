@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(S32WLayout<R, NGR, NSG, NU>::NT, 1)
               for (int q = 0; q < 8; ++q) acc[i][q] = fmaf(xv[q], bv[i], acc[i][q]);
           }
         }
+        fx_reads_done();
         __syncwarp();
         if (lane == 0) fx_mbar_arrive(smem_u32(&gempty[s]));
       }

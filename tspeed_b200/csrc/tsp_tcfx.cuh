@@ -107,6 +107,14 @@ __device__ __forceinline__ void fx_bulk_g2s(uint32_t dst, const void* src, uint3
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
+// Before a warp releases shared memory that it has read by ordinary loads to a
+// bulk copy that will overwrite it: the copy writes through the async proxy,
+// which an mbarrier arrival alone does not order after those loads. Without
+// it a refill now and then overtook the last loads of a stage (one run in
+// twenty of the few-shot step at 2Np = 30 differed in some values).
+__device__ __forceinline__ void fx_reads_done() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 // Bounded wait that also gives up when another role has aborted; false on
 // timeout or abort (a timeout raises the abort flag).
 __device__ __forceinline__ bool fx_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -477,6 +485,7 @@ __global__ void __launch_bounds__(FxCfg<R>::NT, 1) k_step_batched_fx(const StepP
         // The values are in registers: the accumulator slot and the scale
         // entry are free again.
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        fx_reads_done();  // the scale entry is refilled by a bulk copy
         __syncwarp();
         if (lane == 0) {
           fx_mbar_arrive(smem_u32(&bacce[a]));
