@@ -61,20 +61,24 @@ struct RowRingCfg {
   static constexpr int SZ = int(sizeof(BT));
   static constexpr int NPAIR = R / 2;
   static constexpr int W = 4;  // warps of a team: blocks of a row
-  // Columns per chunk: whole columns, multiples of 16 bytes. Large chunks cost
-  // fewer waits and requests per row, small ones leave room for more teams per
-  // SM; measured on 40,000 triangles, FP64 2Np = 42: 14 columns 217 us per
-  // step, 7 columns 304; FP32 2Np = 42: 42 columns 120 us, 14 columns 139;
-  // 2Np = 56: 28 columns 201 us, 14 columns 247; 2Np = 72: 24 columns 436 us,
-  // 12 columns 500; 2Np = 90: 10 columns 577 us, 18 columns (one team) 870.
-  static constexpr int NC = SZ == 8 ? (R == 30 ? 15 : R == 42 ? 14 : R == 56 ? 14 : R == 72 ? 12 : R == 90 ? 10 : R)
-                                    : (R == 42 ? 42 : R == 56 ? 28 : R == 72 ? 24 : R == 90 ? 10 : R);
+  // Columns per chunk (whole columns, multiples of 16 bytes), slots per warp
+  // (whole blocks of DEPTH rows ahead, or a part of a block) and teams per SM.
+  // Large chunks cost fewer waits and requests per row; small ones, or a
+  // single slot, leave room for more teams. Measured on 40,000 triangles, us
+  // per step (columns, slots, teams): FP64 2Np = 30 (15, 2, 5) 119, (30, 1, 6)
+  // 116; 42 (14, 3, 3) 208, (6, 7, 3) 291; 56 (14, 2, 3) 437, (28, 2, 2) 420;
+  // 72 (12, 2, 3) 747, (24, 3, 1) 855; 90 (10, 3, 2) 1162, (6, 3, 3) 1313.
+  // FP32 30 (30, 2, 5) 69.9, (30, 1, 7) 62.6; 42 (42, 2, 3) 122, (14, 3, 6)
+  // 119, (42, 1, 5) 117; 56 (14, 4, 3) 272, (28, 2, 3) 200; 72 (12, 3, 4) 445,
+  // (36, 2, 2) 402; 90 (18, 5, 1) 864, (10, 3, 4) 562.
+  static constexpr bool F64 = SZ == 8;
+  static constexpr int NC = F64 ? (R == 42 ? 14 : R == 56 ? 28 : R == 72 ? 12 : R == 90 ? 10 : R)
+                                : (R == 56 ? 28 : R == 72 ? 36 : R == 90 ? 10 : R);
   static constexpr int NCH = R / NC;    // chunks per block
   static constexpr int CB = NC * R * SZ;
   static_assert(R % NC == 0 && CB % 16 == 0, "whole chunks, multiples of 16 bytes");
-  // Slots per warp: whole blocks of DEPTH rows ahead, or a part of a block.
-  static constexpr int NS = SZ == 8 ? (R == 56 ? 2 : R == 72 ? 2 : R == 90 ? 3 : R <= 20 ? 2 : NCH)
-                                    : (R == 72 ? 3 : R == 90 ? 3 : R <= 42 && NCH == 1 ? 2 : NCH);
+  static constexpr int NS = R <= 20 ? 2 : F64 ? (R == 42 ? 3 : R == 56 ? 2 : R == 72 ? 2 : R == 90 ? 3 : 1)
+                                          : (R == 56 ? 2 : R == 72 ? 2 : R == 90 ? 3 : 1);
   static constexpr int DEPTH = NS >= NCH ? NS / NCH : 1;
   static constexpr int LAP = NS >= NCH ? 1 : NCH / NS;  // uses of a slot per block
   static_assert(NS >= NCH ? NS % NCH == 0 : NCH % NS == 0, "a chunk's slot is known at compile time");
@@ -93,7 +97,8 @@ struct RowRingCfg {
   static constexpr size_t smem_bytes() { return size_t(W) * (PER + NS * 8) + YB + W * 3 * 8 + 16; }
   static constexpr int fit() {
     const int n = int((228 * 1024) / (smem_bytes() + 1024));
-    return R <= 30 ? (n > 5 ? 5 : n) : (n > 4 ? 4 : n);
+    const int most = R <= 20 ? 7 : R == 30 ? (F64 ? 6 : 7) : R == 42 && !F64 ? 5 : 4;
+    return n > most ? most : n;
   }
   static constexpr int CTAS = fit();  // per SM
 };
