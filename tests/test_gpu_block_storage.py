@@ -144,6 +144,35 @@ def test_matrix_free_tiles(N, nx, ny):
         assert rel(a[i], b[i]) < 1e-11
 
 
+# Operators just above the size from which the teams claim their rows, against
+# the matrix-free operator (bounds as above and in test_matrix_free_tiles).
+@pytest.mark.parametrize("N,nx,ny,precision", [(6, 76, 75, "fp64"), (6, 112, 100, "fp32"), (7, 84, 80, "fp32"),
+                                               (8, 68, 64, "fp32")])
+def test_claimed_rows(N, nx, ny, precision):
+    m = W.jittered_rect(nx, ny, 100.0 * nx, 100.0 * ny, seed=N)
+    rng = np.random.default_rng(N)
+    vp = 2500 + 1500 * rng.random(m.ne)
+    lam, mu, rho = W.lame(vp, vp / 1.8, 2000 + 500 * rng.random(m.ne))
+    x = rng.standard_normal(m.ne * (N + 1) * (N + 2))
+    out = []
+    for op, prec in (("matrix_free", "fp64"), ("explicit", precision)):
+        with capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(40.0, 30.0)], [(61.0, 33.0), (20.0, 55.0)],
+                                    penalty=10.0, op=op, precision=prec) as s:
+            s.set_dt(1e-5)
+            s.set_ricker(0, 20.0, 0.05, -1e9, 1, 20)
+            y, lmax = s.apply(x), s.estimate_lmax(10)
+            s.set_initial(0, 1e-3 * x)
+            s.enable_energy(True)
+            s.first_step()
+            s.run(9)
+            out.append((y, s.u(), s.seismograms(0, 10), s.energy(1, 9), lmax))
+    a, b = out
+    tol = 1e-11 if precision == "fp64" else 1e-4
+    for i in range(4):
+        assert rel(b[i], a[i]) < tol
+    assert abs(b[4] - a[4]) < tol * a[4]
+
+
 def test_large_read_back_matches_small_ones():
     """Copies of several megabytes pass through the pinned pieces, small ones
     do not: wrapped seismogram rings with rows above one 8 MiB piece, many

@@ -97,7 +97,8 @@ struct tsp_handle {
   int* d_Xex[2] = {nullptr, nullptr};
   // [0] set by a kernel whose bounded wait gave up; [1] set by a step kernel
   // that wrote a NaN or infinite displacement (cleared by new initial values
-  // or a resumed state).
+  // or a resumed state); [2], [3] row counter of the single-shot ring kernel,
+  // one launch of which is in work at a time.
   int* d_err = nullptr;
   int num_sms = 148;
   long long* d_step = nullptr;
@@ -566,8 +567,8 @@ int finish_create(tsp_handle* h) {
   if (h->fx && (rc = fx_dispatch(h, true, 0))) return rc;
   if ((rc = dalloc(h, &h->d_step, 1))) return rc;
   TSP_CUDA(h, cudaMemsetAsync(h->d_step, 0, sizeof(long long), h->stream));
-  if ((rc = dalloc(h, &h->d_err, 2))) return rc;
-  TSP_CUDA(h, cudaMemsetAsync(h->d_err, 0, 2 * sizeof(int), h->stream));
+  if ((rc = dalloc(h, &h->d_err, 4))) return rc;
+  TSP_CUDA(h, cudaMemsetAsync(h->d_err, 0, 4 * sizeof(int), h->stream));
   if ((rc = dalloc(h, &h->d_acc, 3))) return rc;
   if ((rc = upload(h, &h->d_src_elem, h->src_elem.data(), h->src_elem.size()))) return rc;
   {
@@ -934,6 +935,7 @@ int launch_rowring(tsp_handle* h, const tsp::StepParams& p0, cudaStream_t st) {
   tsp::StepParams p = p0;
   p.rows = h->d_rows;
   p.nphys = int(h->nstored);
+  p.row_counter = size_t(h->nstored) * R * R * sizeof(BT) > tsp::row_queue_bytes ? h->d_err + 2 : nullptr;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(unsigned(std::min<long long>(p.ne, (long long)CF::CTAS * h->num_sms)));
   lc.blockDim = dim3(CF::W * 32);

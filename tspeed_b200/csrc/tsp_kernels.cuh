@@ -93,6 +93,9 @@ struct StepParams {
   // number of stored blocks.
   const void* rows;
   int nphys;
+  // [2] rows claimed beyond the teams' first ones, teams done (both zero
+  // between launches); null: the rows are shared out.
+  int* row_counter;
 };
 
 // Gather indices of the step kernels -- row extents, neighbour ids, source

@@ -56,6 +56,12 @@ struct alignas(32) RowRefs {
   } q[4];
 };
 
+// Bytes of stored blocks from which the rows are claimed instead of shared
+// out: five times L2. us per step at 12,000 triangles, shared out / claimed:
+// FP32 2Np = 72 (0.62 GB) 117 / 121, FP64 56 (0.75 GB) 116 / 112, FP32 90
+// (0.97 GB) 156 / 150.
+constexpr size_t row_queue_bytes = size_t(640) << 20;
+
 template <int R, typename BT>
 struct RowRingCfg {
   static constexpr int SZ = int(sizeof(BT));
@@ -94,7 +100,18 @@ struct RowRingCfg {
   static constexpr int XB = ((R * int(sizeof(typename AccOf<BT>::type)) + 15) / 16) * 16;
   static constexpr int PER = NS * CB + XB;                   // one warp: ring and x of its block
   static constexpr int YB = 4 * W * R * 8;                   // row sums of four rows
-  static constexpr size_t smem_bytes() { return size_t(W) * (PER + NS * 8) + YB + W * 3 * 8 + 16; }
+  // Rows claimed as teams come free (see the row queue in the kernel), where
+  // the blocks are of several times the size of L2 (row_queue_bytes). us per
+  // step with a fixed share of rows / claimed, 40,000 triangles: FP64 2Np = 56
+  // 427 / 363, 72 761 / 607; FP32 56 202 / 200, 72 404 / 391, 90 569 / 486;
+  // 120,000 triangles: FP64 56 1445 / 1144, 72 2642 / 2110, FP32 56 663 / 602,
+  // 90 1882 / 1695. Smaller rows lose: FP64 30 115 / 157, 42 215 / 221, FP32
+  // 30 64 / 73, 42 117 / 117.
+  static constexpr bool QUEUE = R >= 56;
+  static constexpr int LOOK = DEPTH + 2;
+  static constexpr int CLAIM = LOOK + 4;
+  static_assert(!QUEUE || CLAIM <= 8, "queue of 16 rows");
+  static constexpr size_t smem_bytes() { return size_t(W) * (PER + NS * 8) + YB + W * 3 * 8 + 16 + (QUEUE ? 16 * 4 : 0); }
   static constexpr int fit() {
     const int n = int((228 * 1024) / (smem_bytes() + 1024));
     const int most = R <= 20 ? 7 : R == 30 ? (F64 ? 6 : 7) : R == 42 && !F64 ? 5 : 4;
@@ -149,18 +166,39 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
   double* red = ysum + 4 * W * R;                                               // [W][3]
   uint64_t* bars = reinterpret_cast<uint64_t*>(red + W * 3) + warp * NS;
   volatile int* abort_s = reinterpret_cast<volatile int*>(reinterpret_cast<uint64_t*>(red + W * 3) + W * NS);
+  volatile int* rowq = abort_s + 4;  // [16]
   const uint32_t ring_a = smem_u32(mine), bar_a = smem_u32(bars);
 
-  const int ne = p.ne, stride = int(gridDim.x);
+  const int ne = p.ne, grid = int(gridDim.x);
   const RowRefs* rows = reinterpret_cast<const RowRefs*>(p.rows);
 
+  // Row queue: the team's first CLAIM rows are blockIdx + k grid, the later
+  // ones are claimed from a counter by the warp whose turn it is, CLAIM rows
+  // ahead. The rows in work then stay close together over the whole chip; with
+  // a fixed share the teams drift apart and the second use of a block misses
+  // L2. Entry n is written by turn n - CLAIM and read from row n - LOOK = n -
+  // CLAIM + 4 on, before which every warp has met that turn (its own turn lies
+  // in between). It is written again at turn n + 16 - CLAIM, when all warps
+  // have come past row n. Claims are made in turn, so once one of them is
+  // behind the last row, all later ones are.
+  if (CF::QUEUE && threadIdx.x < 16) {
+    const long long r = (long long)blockIdx.x + (long long)threadIdx.x * grid;
+    rowq[threadIdx.x] = int(threadIdx.x) < CF::CLAIM && r < ne ? int(r) : ne;
+  }
+  const bool claiming = CF::QUEUE && p.row_counter != nullptr && (long long)CF::CLAIM * grid < ne;
+  // Row number n of the team, ne behind its last.
+  auto row_at = [&](int n) {
+    if constexpr (CF::QUEUE) return int(rowq[n & 15]);
+    const long long r = (long long)blockIdx.x + (long long)n * grid;
+    return r < ne ? int(r) : ne;
+  };
   if (threadIdx.x == 0) *abort_s = 0;
   if (lane == 0) {
     for (int i = 0; i < NS; ++i) fx_mbar_init(bar_a + 8 * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // The warp's block of row e: column and reference, -1 where there is none.
-  auto entry = [&](long long e, int& col, int& ref) {
+  auto entry = [&](int e, int& col, int& ref) {
     col = ref = -1;
     if (e < ne) {
       const int2 v = __ldg(reinterpret_cast<const int2*>(&rows[e].q[warp]));
@@ -174,10 +212,11 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
 #endif
     }
   };
+  if constexpr (CF::QUEUE) __syncthreads();
   int col[DEPTH + 2], ref[DEPTH + 2];  // rows i .. i + DEPTH + 1 of this team
 #pragma unroll
-  for (int d = 0; d < DEPTH + 2; ++d) entry((long long)blockIdx.x + (long long)d * stride, col[d], ref[d]);
-  __syncthreads();
+  for (int d = 0; d < DEPTH + 2; ++d) entry(row_at(d), col[d], ref[d]);
+  if constexpr (!CF::QUEUE) __syncthreads();
 
   auto block_at = [&](int rf) {
     return reinterpret_cast<const unsigned char*>(p.blocks) + size_t(unsigned(rf) >> 1) * size_t(R * R * CF::SZ);
@@ -234,7 +273,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     }
   };
   const double xsc_all = p.mode == kModePower && p.mesh_of == nullptr ? power_scale(p, 0) : 1.0;
-  int e = blockIdx.x;
+  int e = row_at(0);
 #pragma unroll
   for (int s = 0; s < PPL; ++s) xv[s] = make_double2(0.0, 0.0);
   if (e < ne && !off) {
@@ -247,7 +286,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
   uint32_t phase = 0;  // bit d: phase of the slots that rows i = d (mod DEPTH) use
   bool dead = off;
   int i = 0;
-  for (; e < ne && !off; e = ne - e > stride ? e + stride : ne, ++i) {
+  for (; e < ne && !off; e = row_at(++i)) {
     const int d = DEPTH > 1 ? i % DEPTH : 0;
     double xsc = 1.0;
     if (p.mode == kModePower) {
@@ -269,7 +308,7 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     __syncwarp();
     fetch_x(col[1]);
     int col_l, ref_l;
-    entry((long long)e + (long long)(DEPTH + 2) * stride, col_l, ref_l);
+    entry(row_at(i + CF::LOOK), col_l, ref_l);
 
     double* y = ysum + ((i & 3) * W + warp) * R;
     const int cur = col[0], cref = ref[0];
@@ -417,6 +456,8 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     const bool turn = warp == (i & (W - 1));
     row_barrier(i & 3, turn);
     if (turn) {
+      int claimed = ne;
+      if (claiming && lane == 0) claimed = atomicAdd(p.row_counter, 1);
       // ---- epilogue: inverse mass, leap-frog, source ----
       double* yr = ysum + (i & 3) * W * R;
       const bool is_src = srow >= 0 && k < p.nF;
@@ -492,8 +533,13 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
           atomicAdd(acc3 + 2, a2);
         }
       }
+      if (CF::QUEUE && lane == 0)
+        rowq[(i + CF::CLAIM) & 15] = claiming && claimed < ne - CF::CLAIM * grid ? CF::CLAIM * grid + claimed : ne;
     }
-    if (warp == ((i + 1) & (W - 1)) && ne - e > stride) fetch_row(e + stride);
+    if (warp == ((i + 1) & (W - 1))) {
+      const int en = row_at(i + 1);
+      if (en < ne) fetch_row(en);
+    }
 #pragma unroll
     for (int t = 0; t < DEPTH + 1; ++t) {
       col[t] = col[t + 1];
@@ -535,7 +581,14 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
     if (p.mode == kModePower) atomicAdd(p.acc + threadIdx.x, t);
     else atomicAdd(p.energy + (k % p.energy_cap), t);
   }
-  if (threadIdx.x == 0 && *abort_s) atomicExch(err_flag, 1);
+  if (threadIdx.x == 0) {
+    if (*abort_s) atomicExch(err_flag, 1);
+    // The last team to end clears the counters for the next launch.
+    if (claiming && atomicAdd(p.row_counter + 1, 1) == grid - 1) {
+      p.row_counter[0] = 0;
+      p.row_counter[1] = 0;
+    }
+  }
 }
 
 }  // namespace tsp
