@@ -1539,16 +1539,15 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
   if (h->op_kind == TSP_OP_MATRIX_FREE) {
     const std::vector<double> pk = matfree_tables(P->N, T);
     double *d_tab = nullptr, *d_alpha = nullptr, *d_face = nullptr;
-    int* d_nbr = nullptr;
     const size_t nd = size_t(h->ne) * 3 * T.Q * 4;
     if ((rc = upload(h, &d_tab, pk.data(), pk.size())) || (rc = dalloc(h, &d_alpha, size_t(h->ne) * 10)) ||
-        (rc = dalloc(h, &d_face, size_t(h->ne) * 36)) || (rc = dalloc(h, &d_nbr, size_t(h->ne) * 3)) ||
+        (rc = dalloc(h, &d_face, size_t(h->ne) * 36)) ||
         (rc = dalloc(h, &h->d_D[0], nd)) || (rc = dalloc(h, &h->d_D[1], nd)))
       return create_error_from(h, rc);
     for (int i = 0; i < 2; ++i) TSP_CUDA(h, cudaMemsetAsync(h->d_D[i], 0, nd * sizeof(double), h->stream));
     tsp::k_matfree_geometry<<<(h->ne + 127) / 128, 128, 0, h->stream>>>(h->ne, d_invJ, d_detJ, d_lam, d_mu, d_elen,
                                                                         d_enrm, d_neigh, d_nedge,
-                                                                        P->penalty * h->N * h->N, d_alpha, d_face, d_nbr);
+                                                                        P->penalty * h->N * h->N, d_alpha, d_face);
     cudaError_t ge = cudaGetLastError();
     if (ge == cudaSuccess) ge = cudaStreamSynchronize(h->stream);
     if (ge != cudaSuccess) {
@@ -1558,7 +1557,6 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
     h->mf.tables = d_tab;
     h->mf.alpha = d_alpha;
     h->mf.face = d_face;
-    h->mf.nbr = d_nbr;
     for (void* q : {(void*)d_neigh, (void*)d_nedge, (void*)d_invJ, (void*)d_detJ, (void*)d_elen, (void*)d_enrm,
                     (void*)d_lam, (void*)d_mu})
       dfree(h, q);

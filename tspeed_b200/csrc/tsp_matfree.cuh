@@ -17,14 +17,17 @@
 // m8n8k4.f64 (exact FP64 products, FP64 accumulation): the table fragment is
 // the A operand, stored in fragment order in shared memory, and the tile's two
 // displacement components are two B operands that share it. Measured, us per
-// step before (one warp per element on the CUDA cores, neighbours' traces
-// recomputed, tables read element by element) and now: 160,000 triangles N = 6
-// 1146 -> 260, 40,000 triangles N = 4 153 -> 35, N = 8 579 -> 172; 6,734
-// triangles N = 3 24.9 -> 8.4. Bound: the FP64 tensor rate (478 MMAs per tile
-// at N = 6: 132 us for 160,000 triangles; the pipe is busy half of the time)
-// and the latency of a tile's loads. Twelve warps per SM: sixteen spill at
-// N = 6 (285 us). L2 prefetches of the next tile did not help (N = 5 186 us
-// against 177).
+// step with one warp per element on the CUDA cores (neighbours' traces
+// recomputed, tables read element by element) / now: 160,000 triangles N = 6
+// 1146 / 249; 40,000 triangles N = 4 153 / 32, N = 8 579 / 169; 6,734 triangles
+// N = 3 24.9 / 7.9. Bound: the FP64 tensor rate (478 MMAs per tile at N = 6:
+// 132 us for 160,000 triangles; the pipe is busy half of the time) and the
+// latency of a tile's loads, of which
+// two rounds are left: what a tile starts with (face records, neighbours,
+// inverse masses) is copied to shared memory a tile ahead (N = 6 262 without),
+// every edge value is requested at once. Twelve warps per SM: sixteen spill at
+// N = 6 (285 us); coefficients requested a tile ahead, or edge values in flight
+// during the volume term, spill too (272 to 318 us).
 //
 // The face values are the step's only coupling between elements: every
 // element keeps u and T at its 3Q edge points (four values each) beside its
@@ -42,14 +45,16 @@
 #include <stdint.h>
 
 #include "tsp_kernels.cuh"
+#include "tsp_tcgen05.cuh"
 
 namespace tsp {
 
 struct MatFreeParams {
   const double* tables;  // fragment-ordered volume, lift and trace tables (MFCfg)
   const double* alpha;   // [ne][10] |detJ| alpha: (00: 00 01 11) (11: 00 01 11) (01: 00 01 10 11)
-  const double* face;    // [ne][3][12]: pen N^2 (c00, c01, c11), 0, L/2 beta^{mn}_a [m][n][a]
-  const int* nbr;        // [ne][3] 4 * neighbour + its face, -1 on the boundary
+  // [ne][3][12]: pen N^2 (c00, c01, c11), 4 * neighbour + its face (a whole
+  // number's bits, -1 on the boundary), L/2 beta^{mn}_a [m][n][a]
+  const double* face;
   const double* din;     // [ne][3Q][4] u^0, u^1, T^0, T^1 of u^k at the edge points
   double* dout;          // the same of u^{k+1}; null: not wanted
 };
@@ -72,13 +77,16 @@ struct MFCfg {
   static constexpr int TABLES = VOL + LIFT + TRC;
   // Per warp: rows of eight elements (fluxes, then u^{k+1}), face records.
   static constexpr int ROWS = 4 * KL > 8 * MT ? 4 * KL : 8 * MT;
-  static constexpr int FP = 38;                 // pitch of an element's face records
-  static constexpr int WS = 2 * ROWS * 8 + 8 * FP;
-  static constexpr int warps() {
-    const int n = (227 * 1024 / 8 - TABLES) / (WS + 1);
+  static constexpr int FP = 38;                 // pitch of an element's face records; its inverse mass at 36
+  static constexpr int warps(int fb) {
+    const int n = (227 * 1024 / 8 - TABLES) / (2 * ROWS * 8 + fb * 8 * FP + 1);
     return N <= 4 ? 8 : n > 12 ? 12 : n;
   }
-  static constexpr int WARPS = warps();
+  // The next tile's records are requested a tile ahead where a second buffer
+  // costs no warp.
+  static constexpr int FB = warps(2) == warps(1) ? 2 : 1;
+  static constexpr int WS = 2 * ROWS * 8 + FB * 8 * FP;
+  static constexpr int WARPS = warps(FB);
   static constexpr size_t smem_bytes() { return size_t(TABLES + WARPS * WS + WARPS) * sizeof(double); }
   static constexpr int fit() {
     int n = int(228 * 1024 / (smem_bytes() + 1024));
@@ -96,7 +104,7 @@ __global__ void k_matfree_geometry(int ne, const double* __restrict__ invJ, cons
                                    const double* __restrict__ lam_, const double* __restrict__ mu_,
                                    const double* __restrict__ elen, const double* __restrict__ enrm,
                                    const int* __restrict__ neigh, const int* __restrict__ nedge, double pen_n2,
-                                   double* __restrict__ alpha, double* __restrict__ face, int* __restrict__ nbr) {
+                                   double* __restrict__ alpha, double* __restrict__ face) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
     const double lam = lam_[e], mu = mu_[e], adet = fabs(detJ[e]);
     const double* iJ = invJ + 4 * size_t(e);  // iJ[a + 2 k] = invJ(a, k)
@@ -124,27 +132,38 @@ __global__ void k_matfree_geometry(int ne, const double* __restrict__ invJ, cons
       f[0] = pen_n2 * ((h_l + 2 * h_m) * n0 * n0 + 2 * h_m * n1 * n1);
       f[1] = pen_n2 * (h_l * n0 * n1);
       f[2] = pen_n2 * ((h_l + 2 * h_m) * n1 * n1 + 2 * h_m * n0 * n0);
-      f[3] = 0.0;
+      f[3] = __longlong_as_double(nb < 0 ? -1 : 4 * nb + nedge[3 * size_t(e) + l]);
       const double tau[4][2] = {{(lam + 2 * mu) * n0, mu * n1}, {lam * n1, mu * n0}, {mu * n1, lam * n0},
                                 {mu * n0, (lam + 2 * mu) * n1}};
       for (int mn = 0; mn < 4; ++mn)
         for (int a = 0; a < 2; ++a) f[4 + mn * 2 + a] = hL * (tau[mn][0] * iJ[a] + tau[mn][1] * iJ[a + 2]);
-      nbr[3 * size_t(e) + l] = nb < 0 ? -1 : 4 * nb + nedge[3 * size_t(e) + l];
     }
   }
 }
 
-// Face records of the tile's elements into the warp's shared memory.
+// Face records and inverse masses of the tile's elements into the warp's
+// shared memory, in flight until mf_faces_landed.
 template <int N>
-__device__ __forceinline__ void mf_load_faces(const MatFreeParams& q, int e8, int ne, int lane, double* fc) {
+__device__ __forceinline__ void mf_load_faces(const MatFreeParams& q, const double* minv, int e8, int ne, int lane,
+                                              double* fc) {
   const int n2 = min(8, ne - e8) * 18;
-  const double2* src = reinterpret_cast<const double2*>(q.face + 36 * size_t(e8));
+  const double* src = q.face + 36 * size_t(e8);
 #pragma unroll
   for (int i = lane; i < 8 * 18; i += 32) {
-    const double2 v = i < n2 ? __ldg(src + i) : make_double2(0.0, 0.0);
     const int el = i / 18;
-    *reinterpret_cast<double2*>(fc + el * MFCfg<N>::FP + 2 * (i - el * 18)) = v;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     smem_u32(fc + el * MFCfg<N>::FP + 2 * (i - el * 18))),
+                 "l"(i < n2 ? src + 2 * i : q.face), "r"(i < n2 ? 16 : 0)
+                 : "memory");
   }
+  if (minv != nullptr && lane < 8)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(fc + lane * MFCfg<N>::FP + 36)),
+                 "l"(minv + min(e8 + lane, ne - 1))
+                 : "memory");
+}
+__device__ __forceinline__ void mf_faces_landed() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
 }
 
 // Values and tractions at the edge points of the tile's elements from the
@@ -214,13 +233,13 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
   const int tiles = (ne + 7) / 8;
   for (int tile = blockIdx.x + gridDim.x * warp; tile < tiles; tile += gridDim.x * CF::WARPS) {
     const int e8 = tile * 8;
-    mf_load_faces<N>(q, e8, ne, lane, fc);
+    mf_load_faces<N>(q, nullptr, e8, ne, lane, fc);
     for (int i = lane; i < 2 * 4 * CF::KS * 8; i += 32) {
       const int el = i & 7, k = (i >> 3) % (4 * CF::KS), m = (i >> 3) / (4 * CF::KS);
       const int e = min(e8 + el, ne - 1);
       un[m * CF::ROWS * 8 + mf_at(k, el)] = k < NP ? x[size_t(e) * R + m * NP + k] : 0.0;
     }
-    __syncwarp();
+    mf_faces_landed();
     mf_traces<N>(tab, un, fc, e8, ne, lane, q.dout);
     __syncwarp();
   }
@@ -239,7 +258,7 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, tg = lane & 3;
   double* rows = tab + CF::TABLES + warp * CF::WS;  // [2][ROWS][8]
-  double* fc = rows + 2 * CF::ROWS * 8;             // [8][FP]
+  double* fc = rows + 2 * CF::ROWS * 8;             // [FB][8][FP]
   double* red = tab + CF::TABLES + CF::WARPS * CF::WS;
 
   {
@@ -247,21 +266,23 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
     for (int i = threadIdx.x; i < CF::TABLES / 2; i += CF::WARPS * 32)
       reinterpret_cast<double2*>(tab)[i] = __ldg(src + i);
   }
+  const int ne = p.ne, tiles = (ne + 7) / 8, first = blockIdx.x + gridDim.x * warp;
+  if (first < tiles) mf_load_faces<N>(q, p.minv, first * 8, ne, lane, fc);
   __syncthreads();
-  // The tables are constant: they are in place before the previous step ends.
+  // Tables and geometry are constant: they are in place before the previous step ends.
   // The state and the edge values change under this grid until the wait, so
   // they are read by ordinary loads, not through the read-only path.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  const int ne = p.ne;
   const long long k = (p.step_base ? *p.step_base : 0) + p.rel;
   const bool stepping = p.mode == kModeStep || p.mode == kModeFirst;
   double en = 0.0, pw1 = 0.0, pw2 = 0.0;  // energy / power-iteration partials
   double chk = 0.0;  // NaN once a non-finite u^{k+1} was written (inf * 0 and NaN * 0 are NaN)
-  const int tiles = (ne + 7) / 8;
-  for (int tile = blockIdx.x + gridDim.x * warp; tile < tiles; tile += gridDim.x * CF::WARPS) {
-    const int e8 = tile * 8;
+  const int src_e = stepping && p.src_of == nullptr && p.src_elem != nullptr ? src_elem_at(p, 0) : -1;
+  for (int tile = first; tile < tiles; tile += gridDim.x * CF::WARPS) {
+    const int e8 = tile * 8, e8n = (tile + gridDim.x * CF::WARPS) * 8;
+    mf_faces_landed();
     // ---- B fragments of u^k and the element's elastic factors ----
     const int eg = min(e8 + g, ne - 1);
     double xb[KS][2], al[10];
@@ -296,14 +317,12 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
       int nb[3];
 #pragma unroll
       for (int l = 0; l < 3; ++l) {
-        nb[l] = __ldg(q.nbr + 3 * size_t(e) + l);
+        nb[l] = int(__double_as_longlong(fc[el * CF::FP + 12 * l + 3]));
         if (nb[l] >= 0) nb[l] = (TSP_INDEX(nb[l] >> 2, 0, ne, kSiteNeigh) << 2) | (nb[l] & 3);
       }
-      mf_load_faces<N>(q, e8, ne, lane, fc);
-      __syncwarp();
       double xsc = 1.0;
       if (p.mode == kModePower) xsc = power_scale(p, e);
-#pragma unroll 3
+#pragma unroll
       for (int r = lane >> 3; r < RQ; r += 4) {
         const int l = r >= 2 * Q ? 2 : r >= Q ? 1 : 0, kq = r - l * Q;
         const int code = l == 0 ? nb[0] : l == 1 ? nb[1] : nb[2];
@@ -382,6 +401,16 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
           upv[t][m][h] = row && stepping && p.uprev != nullptr ? p.uprev[at + r] : 0.0;
         }
     }
+    int t0 = 0, t1 = 0;
+    if (stepping && p.rcv_ptr != nullptr) {
+      t0 = rcv_ptr_at(p, e8);
+      t1 = rcv_ptr_at(p, min(e8 + 8, ne));
+    }
+    double* fnext = fc;
+    if constexpr (CF::FB == 2) {
+      fnext = (fc - rows) > 2 * CF::ROWS * 8 ? fc - 8 * CF::FP : fc + 8 * CF::FP;
+      if (e8n < ne) mf_load_faces<N>(q, p.minv, e8n, ne, lane, fnext);
+    }
     // ---- lift of the fluxes (w_k is in the table) ----
 #pragma unroll 2
     for (int ks = 0; ks < KL; ++ks) {
@@ -400,10 +429,10 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
       const int el = 2 * tg + h, e = e8 + el;
       const bool in = e < ne;
       const int ec = in ? e : ne - 1;
-      const double mi = p.minv[ec];
+      const double mi = fc[el * CF::FP + 36];
       const double dt = p.dt_elem ? p.dt_elem[ec] : p.dt;
       const int srow = !stepping ? -1 : p.src_of ? p.src_of[ec]
-                                      : ((p.src_elem != nullptr && src_elem_at(p, 0) == ec) ? 0 : -1);
+                                      : src_e == ec ? 0 : -1;
       const bool is_src = srow >= 0 && k < p.nF;
       const double xsc = p.mode != kModePower ? 1.0 : power_scale(p, ec);
       double* og = p.out + size_t(ec) * R;
@@ -472,20 +501,19 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
     }
     __syncwarp();
     // ---- receivers of the tile's elements: sample u^{k+1} ----
-    if (stepping && p.rcv_ptr != nullptr) {
+    if (t1 > t0) {
       const int last = min(e8 + 8, ne);
-      const int t0 = rcv_ptr_at(p, e8), t1 = rcv_ptr_at(p, last);
-      if (t1 > t0) {
-        for (int e = e8; e < last; ++e) {
-          const int r0 = rcv_ptr_at(p, e), r1 = rcv_ptr_at(p, e + 1);
-          sample_receivers<NP>(p, r0, r1, k, 0, lane,
-                               [&](int c, int i) { return rows[c * CF::ROWS * 8 + mf_at(i, e - e8)]; });
-        }
+      for (int e = e8; e < last; ++e) {
+        const int r0 = rcv_ptr_at(p, e), r1 = rcv_ptr_at(p, e + 1);
+        sample_receivers<NP>(p, r0, r1, k, 0, lane,
+                             [&](int c, int i) { return rows[c * CF::ROWS * 8 + mf_at(i, e - e8)]; });
       }
     }
     // ---- edge values of u^{k+1} for the next step ----
     if (q.dout != nullptr) mf_traces<N>(trc, rows, fc, e8, ne, lane, q.dout);
     __syncwarp();
+    if (CF::FB == 1 && e8n < ne) mf_load_faces<N>(q, p.minv, e8n, ne, lane, fc);
+    fc = fnext;
   }
   if (chk != chk && p.nonfinite != nullptr) *p.nonfinite = 1;
   const bool power = p.mode == kModePower && p.mesh_of == nullptr;
