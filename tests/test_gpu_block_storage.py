@@ -110,6 +110,39 @@ def test_few_shots(N, S, symmetric, precision, monkeypatch):
         assert rel(seis[k], sr) < tol[1]
 
 
+# Rows whose diagonal block is not the first, and rows without one: u^k of the
+# update has its own way there.
+@pytest.mark.parametrize("N,S", [(3, 9), (4, 24), (7, 6)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_few_shots_without_diagonal(N, S, precision, monkeypatch):
+    monkeypatch.delenv("TSP_BATCHED_VARIANT", raising=False)
+    ne, Np = 12, (N + 1) * (N + 2) // 2
+    row_ptr, col, blocks, minv = random_operator(ne, N, N + S, False)
+    rp, keep = [0], []
+    for e in range(ne):
+        r = list(range(row_ptr[e], row_ptr[e + 1]))
+        if len(r) > 1:
+            r = r[1:] if e % 3 == 0 else r[1:] + r[:1] if e % 3 == 1 else r
+        keep += r
+        rp.append(len(keep))
+    row_ptr, col, blocks = np.array(rp, np.int32), col[keep], blocks[keep]
+    rng = np.random.default_rng(S)
+    u0 = rng.standard_normal((S, 2 * ne * Np))
+    phi = rng.standard_normal((S, Np))
+    F = rng.standard_normal((S, 3, 2))
+    with capi.Simulation.from_blocks(row_ptr, col, blocks, minv, [5] * S, phi, [4], phi[:1], precision=precision) as s:
+        s.set_dt(0.01)
+        for k in range(S):
+            s.set_force_table(k, F[k])
+            s.set_initial(k, u0[k])
+        s.first_step()
+        s.run(2)
+        u = s.u_all()
+    for k in range(S):
+        ur, _, _ = O.leapfrog(row_ptr, col, blocks, minv, ne, Np, 0.01, 3, 5, phi[k], F[k], [4], phi[:1], u0[k])
+        assert rel(u[k], ur) < (1e-12 if precision == "fp64" else 1e-4)
+
+
 # Element counts around the tile of eight, and more tiles than one round of warps.
 @pytest.mark.parametrize("N", range(1, 9))
 @pytest.mark.parametrize("nx,ny", [(1, 1), (3, 1), (2, 2), (3, 3), (5, 5), (60, 57)])

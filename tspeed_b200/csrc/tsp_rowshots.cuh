@@ -20,8 +20,11 @@
 // B[k][n] at column k, row n of the block, or transposed at column n, row k.
 // Where 2Np is not a multiple of 4 the last k step's padding is masked in both
 // operands; rows past 2Np only reach outputs that are dropped. The epilogue's
-// u^k and u^{k-1} and the next row's references are requested before the
-// products.
+// u^{k-1} and the next row's references are requested before the products; its
+// u^k likewise, or it is read from the state tile of the diagonal block
+// (STAGED): L2 to shared memory carries 37 KB per row of 24 shots at 2Np = 30
+// with FP32 blocks, u^k from memory 5.8 KB more, and 14,520 triangles take
+// 132.0 us per step instead of 144.6.
 //
 // Every ring belongs to one group, in that group's row order, so use j / NSG
 // of a stage is unambiguous for both sides. Every wait is bounded (about a
@@ -73,6 +76,14 @@ struct RowShotsCfg {
   static constexpr int MT = ST / 8;
   static constexpr int NTW = rowshots_tiles(R, ST, sizeof(BT) == 8);
   static constexpr int WN = (NTL + NTW - 1) / NTW;
+  // u^k of the epilogue from the diagonal block's state tile instead of from
+  // memory: less traffic, but read between the wait for the stage and the
+  // products. It pays for the large tiles beside FP32 blocks; 4,900 triangles,
+  // us per step, memory / stage: FP32 24 shots 2Np = 30 51.9 / 47.4, 42 91.4 /
+  // 85.2, 56 126 / 130, 72 202 / 196; 32 shots 56 174 / 169, 72 248 / 251, 90 417 / 397; 16
+  // shots 42 54.7 / 57.7, 56 89 / 95; FP64 24 shots 30 48.7 / 49.0, 90 305 /
+  // 316; 8 shots 72 103 / 107.
+  static constexpr bool STAGED = sizeof(BT) == 4 && ((ST == 32 && R != 72) || (ST == 24 && R != 56));
   static constexpr int BB = R * R * int(sizeof(BT));  // bytes: the block
   static constexpr int XB = ST * R * 8;               // the state tile
   static constexpr int STAGE = BB + XB;
@@ -245,6 +256,8 @@ __global__ void __launch_bounds__(RowShotsCfg<R, ST, BT>::NT, 1) k_step_rowshots
         q1 = rcv_ptr_at(p, e + 1);
       }
       // u^k and u^{k-1} of this lane's outputs, in flight during the products.
+      // STAGED: u^k from memory only where the row has no diagonal block.
+      const bool diag = CF::STAGED && (rr.a.x == e || rr.a.z == e || rr.b.x == e || rr.b.z == e);
       double2 uk[MT][NTW], up[MT][NTW];
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
@@ -254,7 +267,7 @@ __global__ void __launch_bounds__(RowShotsCfg<R, ST, BT>::NT, 1) k_step_rowshots
         for (int q = 0; q < NTW; ++q) {
           const int r0 = (nt0 + q) * 8 + 2 * tg;
           const bool in = sh < nsv && nt0 + q < NTL && r0 < R;
-          uk[mt][q] = in ? *reinterpret_cast<const double2*>(p.x + me + r0) : make_double2(0.0, 0.0);
+          if (!diag) uk[mt][q] = in ? *reinterpret_cast<const double2*>(p.x + me + r0) : make_double2(0.0, 0.0);
           up[mt][q] = in && p.uprev ? *reinterpret_cast<const double2*>(p.uprev + me + r0) : make_double2(0.0, 0.0);
         }
       }
@@ -278,6 +291,15 @@ __global__ void __launch_bounds__(RowShotsCfg<R, ST, BT>::NT, 1) k_step_rowshots
         }
         const BT* B = reinterpret_cast<const BT*>(gst + size_t(s) * CF::STAGE);
         const double* X = reinterpret_cast<const double*>(gst + size_t(s) * CF::STAGE + CF::BB) + gs * R + tg;
+        if (CF::STAGED && cr.x == e) {
+          const double* U = reinterpret_cast<const double*>(gst + size_t(s) * CF::STAGE + CF::BB) + gs * R + 2 * tg;
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int q = 0; q < NTW; ++q)
+              if ((nt0 + q) * 8 + 2 * tg < R)
+                uk[mt][q] = *reinterpret_cast<const double2*>(U + mt * 8 * R + (nt0 + q) * 8);
+        }
         // B[k][n]: column k, row n of the block; transposed: column n, row k.
         const bool tr = cr.y & 1;
         const BT* Bt = B + (tr ? (nt0 * 8 + g) * R + tg : tg * R + nt0 * 8 + g);
