@@ -75,15 +75,24 @@ def captured_traffic(kernel, ne, nshots):
 
 # Batched FP32 step kernels by variant (tsp_get_kernel_variant), for 2Np = 42.
 KERNELS = {0: "k_step_batched32k<42>", 1: "k_step_batched32p<42,64,4>", 2: "k_step_batched32<42>",
-           4: "k_step_batched_fx<42>", 7: "k_step_batched32w<42,3,3,2,1,6>", 8: "k_step_batched32w<42,4,2,2,1,3>"}
+           4: "k_step_batched_fx<42>", 7: "k_step_batched32w<42,3,3,2,1,6>", 8: "k_step_batched32w<42,4,2,2,1,3>",
+           14: "k_step_rowshots<42>"}
+
+
+def ring_kernel(R, precision):
+    """Whether a single-shot explicit handle runs k_step_rowring (else k_step_rows)."""
+    return R >= {"fp64": 20, "fp32": 42}.get(precision, 1 << 30)
 
 
 def bytes_per_step(ne, Np, nnzb, nshots, precision):
-    """Algorithmic HBM bytes of one step: every block once, the state read
-    (u^k, u^{k-1}) and written (u^{k+1}) once per shot, minv once. The
+    """Algorithmic HBM bytes of one step: every stored block once, the state
+    read (u^k, u^{k-1}) and written (u^{k+1}) once per shot, minv once. The
     tensor-core form ("fx") stores each operator entry as three BF16
-    fixed-point slices (6 bytes)."""
+    fixed-point slices (6 bytes). Single-shot handles with larger blocks store
+    one block per face (the operator is symmetric; both rows use it)."""
     R = 2 * Np
+    if nshots == 1 and ring_kernel(R, precision):
+        nnzb = ne + (nnzb - ne) // 2
     bblk = {"fp64": 8, "fp32": 4, "bf16": 2, "fx": 6}[precision]
     extra = nnzb * 4 if precision == "bf16" else 0
     return nnzb * R * R * bblk + extra + nshots * 2 * ne * Np * 24 + ne * 8
@@ -568,7 +577,8 @@ def main():
     algo = bytes_per_step(prob.mesh.ne, prob.Np, sim.nnzb, prob.nshots, form)
     achieved = algo / (ms_step / 1e3) / 1e9
     kernel = (KERNELS.get(variant, "batched") if variant is not None else
-              "k_step_rows<42>" if prob.nshots == 1 else
+              f"k_step_{'rowring' if ring_kernel(2 * prob.Np, args.precision) else 'rows'}<{2 * prob.Np}>"
+              if prob.nshots == 1 else
               D64_KERNELS.get(variant64, "batched") if args.precision == "fp64" else "k_step_batched<42>")
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": Wm,
             "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -579,7 +589,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": (captured_traffic(kernel, prob.mesh.ne, prob.nshots)
                                      if variant is not None else
-                                     captured_traffic("k_step_rows<42,double>", prob.mesh.ne, prob.nshots)
+                                     captured_traffic("k_step_rowring<42,double>", prob.mesh.ne, prob.nshots)
                                      if prob.nshots == 1 and args.precision == "fp64" else None)
                          if prob.N == 5 else None,
                          "traffic_source": "ncu capture (profiles/traffic.json) scaled by element rows",

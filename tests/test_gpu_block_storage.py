@@ -177,10 +177,12 @@ def test_matrix_free_tiles(N, nx, ny):
         assert rel(a[i], b[i]) < 1e-11
 
 
-# Operators just above the size from which the teams claim their rows, against
-# the matrix-free operator (bounds as above and in test_matrix_free_tiles).
-@pytest.mark.parametrize("N,nx,ny,precision", [(6, 76, 75, "fp64"), (6, 112, 100, "fp32"), (7, 84, 80, "fp32"),
-                                               (8, 68, 64, "fp32")])
+# Operators just below and above the size from which the teams claim their rows
+# (more rows than the teams' first ones either way), against the matrix-free
+# operator (bounds as above and in test_matrix_free_tiles).
+@pytest.mark.parametrize("N,nx,ny,precision", [(6, 70, 70, "fp64"), (6, 76, 75, "fp64"), (6, 100, 60, "fp32"),
+                                               (6, 112, 100, "fp32"), (7, 80, 75, "fp32"), (7, 84, 80, "fp32"),
+                                               (8, 64, 60, "fp32"), (8, 68, 64, "fp32")])
 def test_claimed_rows(N, nx, ny, precision):
     m = W.jittered_rect(nx, ny, 100.0 * nx, 100.0 * ny, seed=N)
     rng = np.random.default_rng(N)

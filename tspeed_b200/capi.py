@@ -372,7 +372,8 @@ class Simulation:
         0/1/2 other CUDA-core kernels, 4 tensor-core fixed-point kernel; FP64
         with several shots: 5 and 6 warp-specialised FP64 tensor-core kernels
         (two groups of 8 consumer warps / one group of 16), 3 single-role
-        one, 2 CUDA-core kernel."""
+        one, 2 CUDA-core kernel. Few shots: 5 (FP64) or 14 (FP32), the
+        few-shot kernel on symmetric storage (no trial)."""
         v = C.c_int32()
         _check(lib().tsp_get_kernel_variant(self._h, C.byref(v)), self._h)
         return v.value

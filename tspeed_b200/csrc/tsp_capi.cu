@@ -504,13 +504,14 @@ int upload_rows(tsp_handle* h, const int* row_ptr, const int* col) {
 }
 
 // Single-shot handles with stored blocks advance by the ring kernel on
-// symmetric storage from 2Np = 30 on, FP64 ones from 2Np = 20 on. Below, a row
+// symmetric storage, FP64 from 2Np = 20 on, FP32 from 2Np = 42 on. Below, a row
 // is so short that the ring kernel's work per row, not its bytes, sets the
 // time, and the register-streaming row kernel wins (40,000 triangles, us per
-// step, ring / rows: FP64 2Np = 12 85 / 37, 20 74 / 84, 30 117 / 327; FP32
-// 2Np = 20 65 / 50, 30 70 / 97). BF16 blocks are not multiples of the 16 bytes
+// step, ring / rows: FP64 2Np = 12 85 / 37, 20 75 / 84, 30 116 / 327; FP32
+// 2Np = 20 65 / 50, 42 120 / 183; FP32 30: 6,000 triangles 16.1 / 14.4, 40,000
+// 90 / 97). BF16 blocks are not multiples of the 16 bytes
 // of a bulk copy.
-constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 30); }
+constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 42); }
 // Handles of a few shots use the same storage with shot tiles of 8 to 32
 // (k_step_rowshots), unless TSP_BATCHED_VARIANT asks for a batched kernel.
 // Most shots for which that is the faster one (0: any number), from 4,900
@@ -917,16 +918,17 @@ int launch_ksplit(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   return TSP_OK;
 }
 
-// Single-shot ring kernel: persistent, one team of four warps per CTA, launched with programmatic stream serialization so that a step's rings fill
-// while the previous step ends.
-template <int R, typename BT, bool ORD = false>
+// Single-shot ring kernel: persistent, one team of four warps per CTA, launched
+// with programmatic stream serialization so that a step's rings fill while the
+// previous step ends.
+template <int R, typename BT>
 int launch_rowring(tsp_handle* h, const tsp::StepParams& p0, cudaStream_t st) {
   typedef tsp::RowRingCfg<R, BT> CF;
   constexpr size_t smem = CF::smem_bytes();
   static_assert(CF::CTAS >= 1 && CF::CTAS * (smem + 1024) <= 228 * 1024, "row ring kernel shared memory");
   static unsigned long long configured = 0;
   const unsigned long long bit = 1ull << (h->device & 63);
-  auto kern = tsp::k_step_rowring<R, BT, ORD>;
+  auto kern = tsp::k_step_rowring<R, BT>;
   if (!(configured & bit)) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("row ring kernel smem: ") + cudaGetErrorString(e));
@@ -1003,9 +1005,7 @@ int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
       const bool stepping = p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst;
       if (h->S > 1 && stepping)
         return fp64 ? launch_rowshots_of<R, double>(h, p, st) : launch_rowshots_of<R, float>(h, p, st);
-      return fp64       ? launch_rowring<R, double>(h, p, st)
-             : stepping ? launch_rowring<R, float>(h, p, st)
-                        : launch_rowring<R, float, true>(h, p, st);
+      return fp64 ? launch_rowring<R, double>(h, p, st) : launch_rowring<R, float>(h, p, st);
     }
   }
   if constexpr (R <= 56) {

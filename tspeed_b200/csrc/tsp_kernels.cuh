@@ -273,7 +273,10 @@ struct RowTeam {
 // column order: the same bits either way.
 // Lanes that own two row pairs (2Np > 64) hold twice the loads per column:
 // the cap is halved there, which keeps 2Np = 72 at two CTAs per SM (FP32
-// blocks unrolled by 24 took 136 registers, one CTA).
+// blocks unrolled by 24 took 136 registers, one CTA). Since single-shot
+// handles with larger blocks take the ring kernel (tsp_rowring.cuh), this
+// kernel serves small blocks, BF16, and the single products of handles whose
+// blocks are stored for the batched kernels.
 template <int R, typename BT>
 constexpr int row_unroll() {
   if (sizeof(BT) == 8 && R % 8 == 0) return 8;

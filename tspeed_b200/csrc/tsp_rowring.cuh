@@ -58,8 +58,8 @@ struct alignas(32) RowRefs {
 
 // Bytes of stored blocks from which the rows are claimed instead of shared
 // out: five times L2. us per step at 12,000 triangles, shared out / claimed:
-// FP32 2Np = 72 (0.62 GB) 117 / 121, FP64 56 (0.75 GB) 116 / 112, FP32 90
-// (0.97 GB) 156 / 150.
+// FP32 2Np = 72 (0.62 GB) 131 / 132, FP64 56 (0.75 GB) 117 / 112, FP32 90
+// (0.97 GB) 179 / 164.
 constexpr size_t row_queue_bytes = size_t(640) << 20;
 
 template <int R, typename BT>
@@ -74,9 +74,9 @@ struct RowRingCfg {
   // per step (columns, slots, teams): FP64 2Np = 30 (15, 2, 5) 119, (30, 1, 6)
   // 116; 42 (14, 3, 3) 208, (6, 7, 3) 291; 56 (14, 2, 3) 437, (28, 2, 2) 420;
   // 72 (12, 2, 3) 747, (24, 3, 1) 855; 90 (10, 3, 2) 1162, (6, 3, 3) 1313.
-  // FP32 30 (30, 2, 5) 69.9, (30, 1, 7) 62.6; 42 (42, 2, 3) 122, (14, 3, 6)
-  // 119, (42, 1, 5) 117; 56 (14, 4, 3) 272, (28, 2, 3) 200; 72 (12, 3, 4) 445,
-  // (36, 2, 2) 402; 90 (18, 5, 1) 864, (10, 3, 4) 562.
+  // FP32 (with lane groups over the columns, before ORD) 42 (42, 2, 3) 122,
+  // (14, 3, 6) 119, (42, 1, 5) 117; 56 (14, 4, 3) 272, (28, 2, 3) 200; 72
+  // (12, 3, 4) 445, (36, 2, 2) 402; 90 (18, 5, 1) 864, (10, 3, 4) 562.
   static constexpr bool F64 = SZ == 8;
   static constexpr int NC = F64 ? (R == 42 ? 14 : R == 56 ? 28 : R == 72 ? 12 : R == 90 ? 10 : R)
                                 : (R == 56 ? 28 : R == 72 ? 36 : R == 90 ? 10 : R);
@@ -103,10 +103,10 @@ struct RowRingCfg {
   // Rows claimed as teams come free (see the row queue in the kernel), where
   // the blocks are of several times the size of L2 (row_queue_bytes). us per
   // step with a fixed share of rows / claimed, 40,000 triangles: FP64 2Np = 56
-  // 427 / 363, 72 761 / 607; FP32 56 202 / 200, 72 404 / 391, 90 569 / 486;
-  // 120,000 triangles: FP64 56 1445 / 1144, 72 2642 / 2110, FP32 56 663 / 602,
-  // 90 1882 / 1695. Smaller rows lose: FP64 30 115 / 157, 42 215 / 221, FP32
-  // 30 64 / 73, 42 117 / 117.
+  // 430 / 367, 72 752 / 631; FP32 56 242 / 226, 72 448 / 429, 90 718 / 552;
+  // 120,000 triangles: FP64 56 1439 / 1133, 72 2650 / 2089, FP32 56 799 / 669,
+  // 90 2335 / 1809. Smaller rows lose: FP64 30 115 / 157, 42 211 / 221, FP32
+  // 42 118 / 118.
   static constexpr bool QUEUE = R >= 56;
   static constexpr int LOOK = DEPTH + 2;
   static constexpr int CLAIM = LOOK + 4;
@@ -114,7 +114,7 @@ struct RowRingCfg {
   static constexpr size_t smem_bytes() { return size_t(W) * (PER + NS * 8) + YB + W * 3 * 8 + 16 + (QUEUE ? 16 * 4 : 0); }
   static constexpr int fit() {
     const int n = int((228 * 1024) / (smem_bytes() + 1024));
-    const int most = R <= 20 ? 7 : R == 30 ? (F64 ? 6 : 7) : R == 42 && !F64 ? 5 : 4;
+    const int most = R <= 20 ? 7 : R == 30 ? 6 : R == 42 && !F64 ? 5 : 4;
     return n > most ? most : n;
   }
   static constexpr int CTAS = fit();  // per SM
@@ -146,14 +146,18 @@ __device__ __forceinline__ void row_barrier(int id, bool wait) {
   else row_barrier_id<3>(wait);
 }
 
-// ORD: every row's FP32 products are summed in column order, block by block
-// (the order of k_step_rows), for single products (kModeApply, kModePower) of
-// FP32 operators: their results stay the same to FP64 rounding whichever
-// storage the handle has. The steps take the faster order.
-template <int R, typename BT, bool ORD = false>
+// ORD (FP32 operators): every row's FP32 products are summed in column order,
+// block by block, as k_step_rows does: the results are the same to the bit
+// whichever storage the handle has. The freer order of the FP64 operators
+// (lane groups over columns, columns started at staggered row pairs) is up to
+// 15 % faster with FP32 blocks too (160,000 triangles N = 6 924 us per step
+// against 997), but its rounding errors are other ones, and seismograms came
+// out up to twice as far from 64-bit products.
+template <int R, typename BT>
 __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(const StepParams p, int* err_flag) {
   typedef RowRingCfg<R, BT> CF;
   typedef typename AccOf<BT>::type AT;
+  constexpr bool ORD = !CF::F64;
   constexpr int G = ORD ? 1 : CF::G, PT = ORD ? 1 : CF::PT, JN = ORD ? CF::NPAIR : CF::JN;
   constexpr bool ROT = CF::ROT && !ORD;
   constexpr int NP = R / 2, NPAIR = CF::NPAIR, NC = CF::NC, NCH = CF::NCH, NS = CF::NS, PPL = CF::PPL, W = CF::W;
@@ -533,8 +537,11 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
           atomicAdd(acc3 + 2, a2);
         }
       }
-      if (CF::QUEUE && lane == 0)
-        rowq[(i + CF::CLAIM) & 15] = claiming && claimed < ne - CF::CLAIM * grid ? CF::CLAIM * grid + claimed : ne;
+      if (CF::QUEUE && lane == 0) {
+        long long r = (long long)CF::CLAIM * grid + claimed;
+        if (!claiming) r = (long long)blockIdx.x + (long long)(i + CF::CLAIM) * grid;
+        rowq[(i + CF::CLAIM) & 15] = r < ne ? int(r) : ne;
+      }
     }
     if (warp == ((i + 1) & (W - 1))) {
       const int en = row_at(i + 1);
