@@ -42,3 +42,33 @@ def test_batch_matches_single_meshes(op, precision):
             s.run(n - 1)
             assert rel(us[m], s.u()) < tol
             assert rel(ss[m], s.seismograms(0, n)[0]) < tol
+
+
+# The second shape's operator is above the size from which rows are claimed.
+@pytest.mark.parametrize("N,nx,ny,op,precision", [(3, 30, 20, "matrix_free", "fp64"), (6, 60, 50, "explicit", "fp64"),
+                                                  (6, 60, 100, "explicit", "fp32")])
+def test_estimate_between_queued_steps_leaves_the_run_alone(N, nx, ny, op, precision):
+    """Batch.run returns while its steps are queued; an estimate asked for then
+    works on the same operators, edge values and row counters."""
+    probs = []
+    for i in range(2):
+        m = W.jittered_rect(nx, ny, 20.0 * nx, 20.0 * ny, seed=i)
+        lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+        probs.append(W.Problem(str(i), m, N, lam, mu, rho, [W.Source(10.0 * nx + 1, 10.0 * ny + 1, 200.0, 1e-3, -1e9, 1)],
+                               [(5.0 * nx, 19.0 * ny)], 900))
+    out = []
+    for estimate in (False, True):
+        with capi.Batch(probs, precision=precision, op=op) as b:
+            lmax = b.estimate_lmax(8)
+            b.set_dt(np.full(2, 1e-5))
+            b.set_ricker(900)
+            b.set_seismogram_capacity(900)
+            b.first_step()
+            for n in (400, 300, 199):
+                b.run(n)
+                if estimate:
+                    assert np.allclose(b.estimate_lmax(8), lmax, rtol=1e-10 if precision == "fp64" else 1e-5, atol=0)
+            out.append([b.u(m) for m in range(2)] + [b.seismograms(m, 0, 900) for m in range(2)])
+    assert all(np.any(u) for u in out[0][:2])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)

@@ -98,7 +98,8 @@ struct tsp_handle {
   // [0] set by a kernel whose bounded wait gave up; [1] set by a step kernel
   // that wrote a NaN or infinite displacement (cleared by new initial values
   // or a resumed state); [2], [3] row counter of the single-shot ring kernel,
-  // one launch of which is in work at a time.
+  // one launch of which is in work at a time (all are on one stream; a batch
+  // waits for its own before a group's is used, see batch_begin).
   int* d_err = nullptr;
   int num_sms = 148;
   long long* d_step = nullptr;
@@ -2754,6 +2755,17 @@ void batch_clear_graphs(tsp_batch* b) {
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
   b->graphs.clear();
 }
+// Makes the batch's device current and waits for the steps queued on the batch
+// stream. Every call but tsp_batch_run works on the groups' own streams, which
+// nothing orders after it, and shares buffers with the steps: the states, the
+// force and dt tables, the matrix-free edge values that a single product writes
+// into the buffer of the level to come, and the claimed-row counters.
+int batch_begin(tsp_batch* b) {
+  cudaError_t e = cudaSetDevice(b->device);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  if (e != cudaSuccess) return bfail(b, TSP_ERR_CUDA, std::string("batch stream: ") + cudaGetErrorString(e));
+  return TSP_OK;
+}
 }  // namespace
 
 extern "C" {
@@ -2938,12 +2950,13 @@ int tsp_batch_info(const tsp_batch* b, int32_t* ngroups, int64_t* total_dofs) {
 
 int tsp_batch_estimate_lmax(tsp_batch* b, int32_t iters, double* lmax) {
   if (!b || !lmax || iters < 1) return TSP_ERR_ARG;
-  cudaSetDevice(b->device);
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
   for (size_t g = 0; g < b->groups.size(); ++g) {
     tsp_handle* h = b->groups[g];
     const int nm = h->nmesh;
     std::vector<double> acc(3 * size_t(nm));
-    const int rc = power_iterate(h, nm, iters, acc.data());
+    rc = power_iterate(h, nm, iters, acc.data());
     if (rc) return bfail(b, rc, h->err);
     for (int q = 0; q < nm; ++q) lmax[b->group_meshes[g][q]] = acc[3 * q] / acc[3 * q + 1];
   }
@@ -2954,7 +2967,8 @@ int tsp_batch_set_dt(tsp_batch* b, const double* dt) {
   if (!b || !dt) return TSP_ERR_ARG;
   for (int m = 0; m < b->nmesh; ++m)
     if (!(dt[m] > 0) || !std::isfinite(dt[m])) return bfail(b, TSP_ERR_ARG, "dt must be positive and finite");
-  cudaSetDevice(b->device);
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
   for (size_t g = 0; g < b->groups.size(); ++g) {
     tsp_handle* h = b->groups[g];
     std::vector<double> de(h->ne);
@@ -2975,7 +2989,8 @@ int tsp_batch_set_dt(tsp_batch* b, const double* dt) {
 int tsp_batch_set_ricker(tsp_batch* b, const double* dt, const double* f0, const double* t0, const double* amp,
                          const int32_t* dir, int64_t n) {
   if (!b || !dt || !f0 || !t0 || !amp || !dir || n < 1) return TSP_ERR_ARG;
-  cudaSetDevice(b->device);
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
   for (size_t g = 0; g < b->groups.size(); ++g) {
     tsp_handle* h = b->groups[g];
     // Source rows are the group's meshes in order: a [nmesh][n][2] table.
@@ -2990,7 +3005,6 @@ int tsp_batch_set_ricker(tsp_batch* b, const double* dt, const double* f0, const
     h->d_F = nullptr;
     h->nF = n;
     h->Fhost = F;
-    int rc;
     if ((rc = upload(h, &h->d_F, F.data(), F.size()))) return bfail(b, rc, h->err);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bfail(b, TSP_ERR_CUDA, "force upload failed");
     clear_graphs(h);
@@ -3001,18 +3015,19 @@ int tsp_batch_set_ricker(tsp_batch* b, const double* dt, const double* f0, const
 
 int tsp_batch_set_seismogram_capacity(tsp_batch* b, int64_t nsteps) {
   if (!b || nsteps < 1) return TSP_ERR_ARG;
-  for (tsp_handle* h : b->groups) {
-    int rc = tsp_set_seismogram_capacity(h, nsteps);
-    if (rc) return bfail(b, rc, h->err);
-  }
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
+  for (tsp_handle* h : b->groups)
+    if ((rc = tsp_set_seismogram_capacity(h, nsteps))) return bfail(b, rc, h->err);
   batch_clear_graphs(b);
   return TSP_OK;
 }
 
 int tsp_batch_first_step(tsp_batch* b) {
   if (!b) return TSP_ERR_ARG;
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
   for (tsp_handle* h : b->groups) {
-    int rc;
     if ((rc = tsp_set_initial(h, 0, nullptr, nullptr))) return bfail(b, rc, h->err);
     if ((rc = tsp_first_step(h))) return bfail(b, rc, h->err);
   }
@@ -3085,17 +3100,17 @@ int tsp_batch_run_timed(tsp_batch* b, int64_t nsteps, double* ms) {
 int tsp_batch_get_u(tsp_batch* b, int32_t mesh, double* out) {
   if (!b || !out || mesh < 0 || mesh >= b->nmesh) return TSP_ERR_ARG;
   tsp_handle* h = b->groups[b->mesh_group[mesh]];
-  cudaSetDevice(b->device);
-  cudaStreamSynchronize(b->stream);
-  const int rc = get_shot(h, h->d_U[h->cur] + size_t(b->mesh_first[mesh]) * h->R, b->mesh_ne[mesh], 0, out);
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
+  rc = get_shot(h, h->d_U[h->cur] + size_t(b->mesh_first[mesh]) * h->R, b->mesh_ne[mesh], 0, out);
   return rc ? bfail(b, rc, h->err) : TSP_OK;
 }
 
 int tsp_batch_get_seismograms(tsp_batch* b, int32_t mesh, int64_t k0, int64_t nk, double* out) {
   if (!b || mesh < 0 || mesh >= b->nmesh || k0 < 0 || nk < 0 || (nk > 0 && !out)) return TSP_ERR_ARG;
   tsp_handle* h = b->groups[b->mesh_group[mesh]];
-  cudaSetDevice(b->device);
-  cudaStreamSynchronize(b->stream);
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
   const int nr = b->mesh_nrcv[mesh], r0 = b->mesh_rcv0[mesh];
   if (nr == 0 || nk == 0) return TSP_OK;
   if (nk > h->seis_cap) return bfail(b, TSP_ERR_ARG, "range longer than the seismogram capacity");
@@ -3110,8 +3125,7 @@ int tsp_batch_get_seismograms(tsp_batch* b, int32_t mesh, int64_t k0, int64_t nk
     k += run;
   }
 #ifdef TSP_CHECKED
-  const int rc = check_device_error(h);
-  if (rc) return bfail(b, rc, h->err);
+  if ((rc = check_device_error(h))) return bfail(b, rc, h->err);
 #endif
   return TSP_OK;
 }
