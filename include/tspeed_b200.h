@@ -162,6 +162,11 @@ int tsp_destroy(tsp_handle* h);
  * *abort_raised = 1, TSP_OK, and the device stays usable. */
 int tsp_selftest_bounded_wait(int32_t device, int32_t* completed, int32_t* abort_raised);
 
+/* Self-test of the reporting: sets (1) or clears (0) the flag that a kernel
+ * raises when a bounded wait gives up. While it is set, every call that hands
+ * out computed values of the handle returns TSP_ERR_TIMEOUT. */
+int tsp_selftest_set_timeout(tsp_handle* h, int32_t value);
+
 /* FP64 tensor-core (DMMA) throughput of a device in TFLOP/s, measured by a
  * register-only loop of a few milliseconds: the FP64 roofline denominator
  * that bench.py reports (no counterpart in the reference). */
@@ -353,6 +358,8 @@ int tsp_batch_set_seismogram_capacity(tsp_batch* b, int64_t nsteps);
 int tsp_batch_first_step(tsp_batch* b);
 int tsp_batch_run(tsp_batch* b, int64_t nsteps);
 int tsp_batch_run_timed(tsp_batch* b, int64_t nsteps, double* ms);
+/* tsp_selftest_set_timeout for every group of the batch. */
+int tsp_selftest_batch_set_timeout(tsp_batch* b, int32_t value);
 /* One mesh's displacement (reference layout) and seismograms [k][rcv][2]. */
 int tsp_batch_get_u(tsp_batch* b, int32_t mesh, double* out);
 int tsp_batch_get_seismograms(tsp_batch* b, int32_t mesh, int64_t k0, int64_t nk, double* out);

@@ -104,6 +104,8 @@ SIGNATURES = {
     "tsp_release_cached_memory": (C.c_int, [C.c_int32]),
     "tsp_fp64_tensor_peak": (C.c_int, [C.c_int32, _dp]),
     "tsp_selftest_bounded_wait": (C.c_int, [C.c_int32, _ip, _ip]),
+    "tsp_selftest_set_timeout": (C.c_int, [C.c_void_p, C.c_int32]),
+    "tsp_selftest_batch_set_timeout": (C.c_int, [C.c_void_p, C.c_int32]),
     "tsp_locate_points": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, _dp, C.c_int32, _ip, C.c_int32, _dp, _ip, _dp]),
     "tsp_eval_basis": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, _dp, _dp]),
     "tsp_quadrature_rule": (C.c_int, [C.c_int32, _dp, _dp]),

@@ -1211,7 +1211,9 @@ void dev_to_ref(const tsp_handle* h, int shot, const double* src_all, double* ds
 }
 
 
-// Reports a bounded device-side wait that gave up (after a synchronisation).
+// Reports a bounded device-side wait that gave up. Every call that hands out
+// what a kernel with such waits has written ends with it: the results are void
+// then, and later launches of the handle write nothing.
 int check_device_error(tsp_handle* h) {
 #ifdef TSP_CHECKED
   // Checked build: the first gather index a kernel found out of range since
@@ -1236,7 +1238,7 @@ int check_device_error(tsp_handle* h) {
   if (!h->d_err) return TSP_OK;
   int v = 0;
   TSP_CUDA(h, copy_sync(&v, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  if (v) return fail(h, TSP_ERR_TIMEOUT, "a tensor-core step kernel timed out waiting for its MMAs; results invalid");
+  if (v) return fail(h, TSP_ERR_TIMEOUT, "a kernel gave up a bounded wait (for a copy into its ring or for its tensor-core products); results invalid");
   return TSP_OK;
 }
 
@@ -1413,7 +1415,7 @@ int power_iterate(tsp_handle* h, int nmesh, int iters, double* acc) {
     if (q) dfree(h, q);
   if (rc) return rc;
   if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("power iteration: ") + cudaGetErrorString(e));
-  return TSP_OK;
+  return check_device_error(h);
 }
 
 int create_error_from(tsp_handle* h, int rc) {
@@ -2089,11 +2091,7 @@ int tsp_get_seismograms(tsp_handle* h, int64_t k0, int64_t nk, double* out) {
                                h->stream));
     k += run;
   }
-#ifdef TSP_CHECKED
-  return check_device_error(h);  // the samples are void after an index failure
-#else
-  return TSP_OK;
-#endif
+  return check_device_error(h);
 }
 
 int tsp_enable_energy(tsp_handle* h, int32_t on) {
@@ -2124,7 +2122,7 @@ int tsp_get_energy(tsp_handle* h, int64_t k0, int64_t nk, double* out) {
     k += run;
   }
   TSP_CUDA(h, cudaStreamSynchronize(h->stream));
-  return TSP_OK;
+  return check_device_error(h);
 }
 
 int tsp_get_state(tsp_handle* h, double* u_prev, double* u_cur, int64_t* steps_done, double* last_time) {
@@ -2144,7 +2142,7 @@ int tsp_get_state(tsp_handle* h, double* u_prev, double* u_cur, int64_t* steps_d
   }
   if (steps_done) *steps_done = h->steps_done;
   if (last_time) *last_time = h->last_time;
-  return TSP_OK;
+  return check_device_error(h);
 }
 
 int tsp_set_state(tsp_handle* h, const double* u_prev, const double* u_cur, int64_t steps_done, double last_time) {
@@ -2188,7 +2186,7 @@ int tsp_check_finite(tsp_handle* h, int32_t* bad) {
   *bad = flag ? 1 : 0;
   for (size_t i = 0; i < all.size() && !*bad; ++i)
     if (!std::isfinite(all[i])) *bad = 1;
-  return TSP_OK;
+  return check_device_error(h);
 }
 
 int tsp_apply(tsp_handle* h, const double* x, double* y) {
@@ -2217,7 +2215,7 @@ int tsp_apply(tsp_handle* h, const double* x, double* y) {
                   h->Np * sizeof(double));
   dfree(h, dx);
   dfree(h, dy);
-  return TSP_OK;
+  return check_device_error(h);
 }
 
 int tsp_estimate_lmax(tsp_handle* h, int32_t iters, double* lmax) {
@@ -2576,6 +2574,14 @@ int tsp_selftest_bounded_wait(int32_t device, int32_t* completed, int32_t* abort
   return TSP_OK;
 }
 
+int tsp_selftest_set_timeout(tsp_handle* h, int32_t value) {
+  if (!h) return TSP_ERR_ARG;
+  int rc;
+  if ((rc = begin(h))) return rc;
+  TSP_CUDA(h, copy_sync(h->d_err, &value, sizeof(value), cudaMemcpyHostToDevice, h->stream));
+  return TSP_OK;
+}
+
 int tsp_fp64_tensor_peak(int32_t device, double* tflops) {
   if (!tflops) return fail(nullptr, TSP_ERR_ARG, "null argument");
   int prev = 0, sms = 0;
@@ -2719,7 +2725,7 @@ extern "C" int tsp_estimate_lmax_noalloc(tsp_handle* h, int32_t iters, double* l
     std::swap(da, db);
   }
   *lmax = lam;
-  return TSP_OK;
+  return check_device_error(h);
 }
 
 
@@ -3036,6 +3042,15 @@ int tsp_batch_first_step(tsp_batch* b) {
   return TSP_OK;
 }
 
+int tsp_selftest_batch_set_timeout(tsp_batch* b, int32_t value) {
+  if (!b) return TSP_ERR_ARG;
+  int rc;
+  if ((rc = batch_begin(b))) return rc;
+  for (tsp_handle* h : b->groups)
+    if ((rc = tsp_selftest_set_timeout(h, value))) return bfail(b, rc, h->err);
+  return TSP_OK;
+}
+
 // All groups' steps in one graph, replayed on the batch stream.
 int tsp_batch_run(tsp_batch* b, int64_t nsteps) {
   NvtxRange nvtx_("tsp_batch_run");
@@ -3091,6 +3106,8 @@ int tsp_batch_run_timed(tsp_batch* b, int64_t nsteps, double* ms) {
     if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&f, e0, e1) != cudaSuccess)
       rc = bfail(b, TSP_ERR_CUDA, "batch timing failed");
   }
+  for (tsp_handle* h : b->groups)
+    if (rc == TSP_OK && (rc = check_device_error(h))) bfail(b, rc, h->err);
   *ms = f;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -3103,6 +3120,7 @@ int tsp_batch_get_u(tsp_batch* b, int32_t mesh, double* out) {
   int rc;
   if ((rc = batch_begin(b))) return rc;
   rc = get_shot(h, h->d_U[h->cur] + size_t(b->mesh_first[mesh]) * h->R, b->mesh_ne[mesh], 0, out);
+  if (!rc) rc = check_device_error(h);
   return rc ? bfail(b, rc, h->err) : TSP_OK;
 }
 
@@ -3124,10 +3142,8 @@ int tsp_batch_get_seismograms(tsp_batch* b, int32_t mesh, int64_t k0, int64_t nk
     if (e != cudaSuccess) return bfail(b, TSP_ERR_CUDA, std::string("seismogram read-back: ") + cudaGetErrorString(e));
     k += run;
   }
-#ifdef TSP_CHECKED
-  if ((rc = check_device_error(h))) return bfail(b, rc, h->err);
-#endif
-  return TSP_OK;
+  rc = check_device_error(h);
+  return rc ? bfail(b, rc, h->err) : TSP_OK;
 }
 
 }  // extern "C"
