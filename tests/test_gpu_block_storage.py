@@ -261,3 +261,22 @@ def test_repeated_steps_are_identical(N, nx, ny, S, precision, monkeypatch):
             assert np.array_equal(u, ref)
         # Every shot had the same state and no force: every shot the same result.
         assert np.array_equal(ref, np.tile(ref[0], (S, 1)))
+
+
+def test_window_of_seismogram_rings_above_2_gib():
+    """The shots' rings lie further apart than the largest pitch of a 2-D copy."""
+    m = W.jittered_rect(6, 5, 600.0, 500.0, seed=3)
+    lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+    rcv = [(600.0 * (r + 0.5) / 1500, 490.0) for r in range(1500)]
+    out = []
+    for cap in (16, 90000):
+        with capi.Simulation.create(m.xy, m.tri, 3, lam, mu, rho, [(210.0, 480.0), (390.0, 480.0)], rcv,
+                                    penalty=10.0) as s:
+            s.set_dt(1e-4)
+            for k in range(2):
+                s.set_ricker(k, 200.0, 1e-3, -1e9, 1, 16)
+            s.set_seismogram_capacity(cap)
+            s.first_step()
+            s.run(15)
+            out.append(s.seismograms(4, 12))
+    assert np.any(out[0][0]) and np.any(out[0][1]) and np.array_equal(*out)

@@ -65,6 +65,21 @@ class Staging {
   unsigned char* mem_ = nullptr;
 };
 
+// Queues a copy of `rows` rows of `width` bytes (pitches in bytes) from the
+// device. 2-D copies are documented for pitches up to the device's maximum,
+// 2^31 - 1 bytes; beyond (one shot's seismogram ring may hold more) every row
+// is a copy of its own.
+inline cudaError_t copy_rows(unsigned char* dst, size_t dpitch, const unsigned char* src, size_t spitch, size_t width,
+                             size_t rows, cudaStream_t st) {
+  constexpr size_t kMaxPitch = (size_t(1) << 31) - 1;
+  if (rows > 1 && dpitch <= kMaxPitch && spitch <= kMaxPitch)
+    return cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, rows, cudaMemcpyDeviceToHost, st);
+  cudaError_t e = cudaSuccess;
+  for (size_t r = 0; r < rows && e == cudaSuccess; ++r)
+    e = cudaMemcpyAsync(dst + r * dpitch, src + r * spitch, width, cudaMemcpyDeviceToHost, st);
+  return e;
+}
+
 // Copies `height` rows of `width` bytes (pitches in bytes) from the device,
 // ordered on `st` and complete on return.
 inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t height,
@@ -74,11 +89,12 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
     width *= height;
     height = 1;
   }
+  unsigned char* d = static_cast<unsigned char*>(dst);
+  const unsigned char* s = static_cast<const unsigned char*>(src);
   auto plain = [&]() {
-    cudaError_t e = height == 1 ? cudaMemcpyAsync(dst, src, width, cudaMemcpyDeviceToHost, st)
-                                : cudaMemcpy2DAsync(dst, dpitch, src, spitch, width, height, cudaMemcpyDeviceToHost, st);
-    const cudaError_t s = cudaStreamSynchronize(st);
-    return e == cudaSuccess ? s : e;
+    const cudaError_t e = copy_rows(d, dpitch, s, spitch, width, height, st);
+    const cudaError_t done = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? done : e;
   };
   const size_t total = width * height;
   if (total < (size_t(2) << 20)) return plain();
@@ -91,8 +107,6 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
     size_t width, rows;
   };
   std::vector<Piece> pieces;
-  unsigned char* d = static_cast<unsigned char*>(dst);
-  const unsigned char* s = static_cast<const unsigned char*>(src);
   if (width > Staging::kPiece) {
     for (size_t r = 0; r < height; ++r)
       for (size_t o = 0; o < width; o += Staging::kPiece)
@@ -167,8 +181,7 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
     }
     const Piece& p = pieces[i];
     unsigned char* to = pin + size_t(b) * Staging::kPiece;
-    e = p.rows == 1 ? cudaMemcpyAsync(to, p.src, p.width, cudaMemcpyDeviceToHost, st)
-                    : cudaMemcpy2DAsync(to, p.width, p.src, spitch, p.width, p.rows, cudaMemcpyDeviceToHost, st);
+    e = copy_rows(to, p.width, p.src, spitch, p.width, p.rows, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[b], st);
     if (i > 0) publish(i - 1);
   }
