@@ -6,8 +6,20 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <new>
 
 #include "tsp_readback.h"
+
+// Host allocations fail while the countdown is at zero (below: they never do).
+static int g_allocs_left = -1;
+void* operator new(size_t n) {
+  if (g_allocs_left == 0) throw std::bad_alloc();
+  if (g_allocs_left > 0) --g_allocs_left;
+  if (void* p = std::malloc(n ? n : 1)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 namespace {
 int copies_1d = 0, copies_2d = 0;
@@ -96,6 +108,16 @@ int main() {
   rows(MiB, 2 * GiB + 160, MiB - 16, 4);              // above it: staged, eight rows per piece
   rows(3 * GiB, 2 * GiB + 160, MiB + 16, 3);
   CHECK(copies_2d == n2 && copies_1d == n1 + 3 + 3 + 4 + 3);
+  // The n-th host allocation of a copy and all later ones fail: the copy is
+  // whole, and the pinned buffers are free again for the next one.
+  for (int n = 0; n < 24; ++n) {
+    g_allocs_left = n;
+    rows(4 * MiB, 5 * MiB, 3 * MiB, 9);
+    g_allocs_left = -1;
+    unsigned char* pin = tsp::Staging::get().take();
+    CHECK(pin != nullptr);
+    tsp::Staging::get().give_back();
+  }
   std::puts("read-back checks passed");
   return 0;
 }

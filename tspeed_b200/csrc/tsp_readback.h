@@ -9,7 +9,8 @@
 //
 // The pinned buffers are one set per process (24 MiB, allocated by the first
 // large copy, returned by tsp_release_cached_memory). A copy that finds them
-// taken by another thread, or cannot start a thread, takes the plain path.
+// taken by another thread, or cannot start a thread or get host memory for its
+// bookkeeping, takes the plain path.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -17,8 +18,9 @@
 #include <algorithm>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -98,7 +100,13 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
   };
   const size_t total = width * height;
   if (total < (size_t(2) << 20)) return plain();
-  unsigned char* pin = Staging::get().take();
+  struct Lease {  // the pinned buffers, given back however the copy ends
+    unsigned char* mem = Staging::get().take();
+    ~Lease() {
+      if (mem) Staging::get().give_back();
+    }
+  } lease;
+  unsigned char* pin = lease.mem;
   if (!pin) return plain();
 
   struct Piece {
@@ -107,14 +115,24 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
     size_t width, rows;
   };
   std::vector<Piece> pieces;
-  if (width > Staging::kPiece) {
-    for (size_t r = 0; r < height; ++r)
-      for (size_t o = 0; o < width; o += Staging::kPiece)
-        pieces.push_back({d + r * dpitch + o, s + r * spitch + o, std::min(Staging::kPiece, width - o), 1});
-  } else {
-    const size_t n = Staging::kPiece / width;
-    for (size_t r = 0; r < height; r += n)
-      pieces.push_back({d + r * dpitch, s + r * spitch, width, std::min(n, height - r)});
+  std::vector<int> moved;
+  std::vector<std::thread> threads;
+  const int want = int(std::min<size_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency() / 2)),
+                                        1 + total / (size_t(4) << 20)));
+  try {
+    if (width > Staging::kPiece) {
+      for (size_t r = 0; r < height; ++r)
+        for (size_t o = 0; o < width; o += Staging::kPiece)
+          pieces.push_back({d + r * dpitch + o, s + r * spitch + o, std::min(Staging::kPiece, width - o), 1});
+    } else {
+      const size_t n = Staging::kPiece / width;
+      for (size_t r = 0; r < height; r += n)
+        pieces.push_back({d + r * dpitch, s + r * spitch, width, std::min(n, height - r)});
+    }
+    moved.assign(pieces.size(), 0);
+    threads.reserve(want);
+  } catch (const std::bad_alloc&) {  // no host memory for the bookkeeping
+    return plain();
   }
 
   // ready: pieces whose data is in its buffer; moved[b]: threads done with the
@@ -122,7 +140,6 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
   std::mutex m;
   std::condition_variable cv;
   size_t ready = 0;
-  std::vector<int> moved(pieces.size(), 0);
   int nthreads = 0;
   bool stop = false;
   auto work = [&](int t) {
@@ -147,18 +164,11 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
       if (++moved[i] == n) cv.notify_all();
     }
   };
-  const int want = int(std::min<size_t>(std::max(1u, std::min(8u, std::thread::hardware_concurrency() / 2)),
-                                        1 + total / (size_t(4) << 20)));
-  std::vector<std::thread> threads;
-  threads.reserve(want);
   try {
     for (int t = 0; t < want; ++t) threads.emplace_back(work, t);
-  } catch (const std::system_error&) {
+  } catch (const std::exception&) {  // no thread, or no memory for one: those that started do the work
   }
-  if (threads.empty()) {
-    Staging::get().give_back();
-    return plain();
-  }
+  if (threads.empty()) return plain();
   {
     std::lock_guard<std::mutex> lk(m);
     nthreads = int(threads.size());
@@ -195,7 +205,6 @@ inline cudaError_t read_back(void* dst, size_t dpitch, const void* src, size_t s
   for (std::thread& t : threads) t.join();
   for (cudaEvent_t v : ev)
     if (v) cudaEventDestroy(v);
-  Staging::get().give_back();
   return e;
 }
 
