@@ -176,7 +176,8 @@ int tsp_fp64_tensor_peak(int32_t device, double* tflops);
  * device that keeps freed memory cached for the process, so creating a
  * simulation after destroying another does not pay for multi-GB device
  * allocations again. This returns the cached memory of a device to the
- * driver (after a device synchronisation). */
+ * driver (after a device synchronisation), and the process's pinned read-back
+ * buffers to the system. */
 int tsp_release_cached_memory(int32_t device);
 
 /* Message of the last failing call on this handle (or of the last failing

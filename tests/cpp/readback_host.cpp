@@ -22,11 +22,12 @@ void operator delete(void* p) noexcept { std::free(p); }
 void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 namespace {
-int copies_1d = 0, copies_2d = 0;
+int copies_1d = 0, copies_2d = 0, host_allocs = 0;
 }
 
 extern "C" {
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  ++host_allocs;
   *p = std::malloc(n);
   return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }
@@ -118,6 +119,13 @@ int main() {
     CHECK(pin != nullptr);
     tsp::Staging::get().give_back();
   }
+  // The buffers are allocated by the copy that reaches the bytes they are worth.
+  tsp::Staging::get().release();
+  const int n0 = host_allocs;
+  for (int n = 0; n < 2; ++n) rows(20 * MiB, 20 * MiB, 20 * MiB, 1);
+  CHECK(host_allocs == n0);
+  for (int n = 0; n < 3; ++n) rows(4 * MiB, 5 * MiB, 4 * MiB, 1);
+  CHECK(host_allocs == n0 + 1);
   std::puts("read-back checks passed");
   return 0;
 }
