@@ -6,6 +6,8 @@ Tolerances: FP64 paths differ from the oracle in summation order only,
 operators hold each entry to 2^-24 of itself and, with one shot, sum at most
 4 * 90 FP32 products per row: 360 * 2^-24 = 2.2e-5 bounds the relative error
 of rows without cancellation; 1e-4 covers the few steps taken here."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -280,3 +282,35 @@ def test_window_of_seismogram_rings_above_2_gib():
             s.run(15)
             out.append(s.seismograms(4, 12))
     assert np.any(out[0][0]) and np.any(out[0][1]) and np.array_equal(*out)
+
+
+def test_read_back_without_device_memory():
+    """A wavefield is read without a transposed copy where the device has no
+    room for one; the calls after it do not see the failed allocation."""
+    rt = ctypes.CDLL("libcudart.so.12")
+    m = W.jittered_rect(260, 260, 2600.0, 2600.0, seed=3)  # 135,200 triangles: 97 MB of displacements
+    lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+    ballast = []
+    with capi.Simulation.create(m.xy, m.tri, 8, lam, mu, rho, [(1310.0, 1290.0)], [(1310.0, 1295.0)], penalty=10.0,
+                                op="matrix_free") as s:
+        s.set_dt(1e-6)
+        s.set_ricker(0, 200.0, 0.0, -1e9, 1, 16)
+        s.first_step()
+        s.step()
+        s.run(2)
+        u0 = s.u()
+        try:
+            capi.release_cached_memory(0)
+            for size in (1 << 30, 64 << 20, 4 << 20):
+                p = ctypes.c_void_p()
+                while rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0:
+                    ballast.append(ctypes.c_void_p(p.value))
+            rt.cudaGetLastError()
+            assert np.array_equal(s.u(), u0)
+            s.step()
+            s.run(2)
+            u1 = s.u()
+        finally:
+            for p in ballast:
+                rt.cudaFree(p)
+        assert len(ballast) > 0 and np.array_equal(s.u(), u1) and not np.array_equal(u1, u0)

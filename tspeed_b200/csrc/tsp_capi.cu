@@ -195,6 +195,7 @@ cudaError_t pool_alloc(tsp_handle* h, void** p, size_t bytes) {
   cudaMemPool_t pool = nullptr;
   cudaError_t e = device_pool(h->device, &pool);
   if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes, pool, h->stream);
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here: not by the next launch's check
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   return e;
 }
