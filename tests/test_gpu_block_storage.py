@@ -314,3 +314,33 @@ def test_read_back_without_device_memory():
             for p in ballast:
                 rt.cudaFree(p)
         assert len(ballast) > 0 and np.array_equal(s.u(), u1) and not np.array_equal(u1, u0)
+
+
+# Receivers in one element and over neighbouring ones, around the counts at
+# which a warp turns from one receiver at a time to one per lane, and above 32.
+@pytest.mark.parametrize("per_element", [1, 3, 4, 5, 31, 33, 70])
+@pytest.mark.parametrize("N,precision,op", [(n, "fp64", "matrix_free") for n in range(1, 9)] +
+                         [(n, "fp64", "explicit") for n in range(3, 9)] + [(n, "fp32", "explicit") for n in range(5, 9)])
+def test_receivers_sample_their_element(N, precision, op, per_element):
+    m = W.jittered_rect(5, 3, 500.0, 300.0, seed=N)
+    lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+    rng = np.random.default_rng(per_element)
+    rcv = []
+    for e in (2, 3, 4, 5, 17, m.ne - 1):  # a tile of eight elements, one alone, the last
+        a, b, c = m.xy[m.tri[e]]
+        for _ in range(per_element if e != 4 else 1):
+            s, t = rng.uniform(0.1, 0.45, 2)
+            rcv.append(tuple(a + s * (b - a) + t * (c - a)))
+    rng.shuffle(rcv)
+    Np = (N + 1) * (N + 2) // 2
+    with capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(210.0, 140.0)], rcv, penalty=10.0, precision=precision,
+                                op=op) as sim:
+        sim.set_dt(1e-6)
+        sim.set_initial(0, rng.standard_normal(2 * m.ne * Np))
+        sim.first_step()
+        sim.run(2)
+        u, seis = sim.u().reshape(2, m.ne, Np), sim.seismograms(2, 1)[0, 0]
+        _, _, elem, phi = sim.export_points()
+    ref = np.einsum("ri,cri->rc", phi, u[:, elem])
+    assert len(set(elem)) == 6
+    assert rel(seis, ref) < 1e-13

@@ -111,7 +111,7 @@ struct tsp_handle {
   int* d_rcv_ptr = nullptr;
   int* d_rcv_id = nullptr;
   double* d_rcv_phi = nullptr;
-  double* d_rcv_phi_q = nullptr;  // in the order of d_rcv_id
+  double* d_rcv_phi_t = nullptr;  // [Np][nrcv] in the order of d_rcv_id
   double* d_seis = nullptr;
   long long seis_cap = 0;
   double* d_energy = nullptr;
@@ -286,10 +286,10 @@ int build_receiver_csr(tsp_handle* h) {
   std::vector<double> rphi(h->rcv_phi);
   if (!h->lref_inv.empty()) map_vectors(h->lref_inv, false, h->Np, rphi.data(), h->nrcv);
   if ((rc = upload(h, &h->d_rcv_phi, rphi.data(), rphi.size()))) return rc;
-  std::vector<double> qphi(rphi.size());
+  std::vector<double> tphi(rphi.size());
   for (int q = 0; q < h->nrcv; ++q)
-    std::copy(&rphi[size_t(ids[q]) * h->Np], &rphi[size_t(ids[q]) * h->Np] + h->Np, &qphi[size_t(q) * h->Np]);
-  if ((rc = upload(h, &h->d_rcv_phi_q, qphi.data(), qphi.size()))) return rc;
+    for (int i = 0; i < h->Np; ++i) tphi[size_t(i) * h->nrcv + q] = rphi[size_t(ids[q]) * h->Np + i];
+  if ((rc = upload(h, &h->d_rcv_phi_t, tphi.data(), tphi.size()))) return rc;
   return TSP_OK;
 }
 
@@ -1112,7 +1112,7 @@ int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, d
   p.rcv_ptr = (sample && h->nrcv > 0) ? h->d_rcv_ptr : nullptr;
   p.rcv_id = h->d_rcv_id;
   p.rcv_phi = h->d_rcv_phi;
-  p.rcv_phi_q = h->d_rcv_phi_q;
+  p.rcv_phi_t = h->d_rcv_phi_t;
   p.seis = h->d_seis;
   p.nrcv = h->nrcv;
   p.seis_cap = h->seis_cap;
@@ -2917,11 +2917,11 @@ int tsp_batch_create(const tsp_problem* meshes, int32_t nmesh, tsp_batch** out) 
     dfree(h, h->d_rcv_ptr);
     dfree(h, h->d_rcv_id);
     dfree(h, h->d_rcv_phi);
-    dfree(h, h->d_rcv_phi_q);
+    dfree(h, h->d_rcv_phi_t);
     h->d_rcv_ptr = nullptr;
     h->d_rcv_id = nullptr;
     h->d_rcv_phi = nullptr;
-    h->d_rcv_phi_q = nullptr;
+    h->d_rcv_phi_t = nullptr;
     std::vector<double> ones(ms.size(), 1.0);
     if ((rc = upload(h, &h->d_src_phi, src_phi.data(), src_phi.size())) ||
         (rc = upload(h, &h->d_src_of, src_of.data(), src_of.size())) ||

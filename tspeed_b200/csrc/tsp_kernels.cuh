@@ -57,7 +57,7 @@ struct StepParams {
   const int* rcv_ptr;         // [ne+1] or null
   const int* rcv_id;          // [nrcv] receiver ids ordered by element
   const double* rcv_phi;      // [nrcv][Np] by receiver id
-  const double* rcv_phi_q;    // [nrcv][Np] in the order of rcv_id
+  const double* rcv_phi_t;    // [Np][nrcv] in the order of rcv_id
   double* seis;               // [S][cap][nrcv][2]
   int nrcv;
   long long seis_cap;
@@ -160,33 +160,61 @@ __device__ __forceinline__ double power_scale(const StepParams& p, int e) {
   return p.xscale_mesh ? p.xscale_mesh[p.mesh_of[e]] : p.xscale;
 }
 
-// Receivers [q0, q1) of one element sampled by a whole warp: lanes share the
-// modes, y(c, i) is mode i of component c of the new level. (One lane per
-// receiver and component walked its modes with a dependent load each: 1.4 us
-// of the 11 us step of 1,600 triangles at N = 4 with 8 receivers, 10 us of
-// 255 at 40,000 triangles, N = 5 with 128.)
-template <int NP, class Y>
+// Receivers [q0, q1) sampled by a whole warp; elem(q) names the element of
+// receiver position q for y(elem, c, i), mode i of component c of its new level.
+// Few receivers: the lanes share the modes of one after the other, 0.23 us
+// each, the latency of a load and of the sums. More: every lane owns a receiver
+// and walks its modes in NP / UN rounds of loads, coalesced over the lanes (the
+// table is [mode][position]); a round takes about as long as one receiver the
+// other way, so the line lies at as many receivers as rounds, three at least.
+// One way for all, us per step on 800 triangles, one receiver after the other /
+// as here: 500 in one element N = 5 FP64 blocks 123 / 17, matrix-free 155 / 21;
+// 2,000 on a line N = 5 matrix-free 94 / 12.5; 16 in one element 10.4 / 7.2.
+// UN: modes whose factors are in flight at once, a divisor of NP (registers).
+template <int NP, int UN, class E, class Y>
 __device__ __forceinline__ void sample_receivers(const StepParams& p, int q0, int q1, long long k, int sh, int lane,
-                                                 Y y) {
+                                                 E elem, Y y) {
   const long long slot = k % p.seis_cap;
-  for (int q = q0; q < q1; ++q) {
-    const int rid = rcv_id_at(p, q);
-    double v0 = 0.0, v1 = 0.0;
+  double* out = p.seis + (size_t(sh) * p.seis_cap + slot) * p.nrcv * 2;
+  if (q1 - q0 <= (NP / UN > 3 ? NP / UN : 3)) {
+    for (int q = q0; q < q1; ++q) {
+      const int el = elem(q), rid = rcv_id_at(p, q);
+      double v0 = 0.0, v1 = 0.0;
 #pragma unroll
-    for (int i = 0; i < NP; i += 32)
-      if (i + lane < NP) {
-        const double ph = __ldg(p.rcv_phi_q + size_t(q) * NP + i + lane);
-        v0 = fma(ph, y(0, i + lane), v0);
-        v1 = fma(ph, y(1, i + lane), v1);
+      for (int i = 0; i < NP; i += 32)
+        if (i + lane < NP) {
+          const double ph = __ldg(p.rcv_phi_t + size_t(i + lane) * p.nrcv + q);
+          v0 = fma(ph, y(el, 0, i + lane), v0);
+          v1 = fma(ph, y(el, 1, i + lane), v1);
+        }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+        v1 += __shfl_xor_sync(0xffffffffu, v1, o);
       }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-      v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+      if (lane == 0) *reinterpret_cast<double2*>(out + 2 * size_t(rid)) = make_double2(v0, v1);
     }
-    if (lane == 0)
-      *reinterpret_cast<double2*>(p.seis + ((size_t(sh) * p.seis_cap + slot) * p.nrcv + rid) * 2) = make_double2(v0, v1);
+    return;
   }
+  static_assert(NP % UN == 0, "whole rounds of modes");
+  for (int q = q0 + lane; q < q1; q += 32) {
+    const int el = elem(q), rid = rcv_id_at(p, q);
+    const double* ph = p.rcv_phi_t + q;
+    double v0 = 0.0, v1 = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < NP; i += UN) {
+      double f[UN];
+#pragma unroll
+      for (int t = 0; t < UN; ++t) f[t] = __ldg(ph + size_t(i + t) * p.nrcv);
+#pragma unroll
+      for (int t = 0; t < UN; ++t) {
+        v0 = fma(f[t], y(el, 0, i + t), v0);
+        v1 = fma(f[t], y(el, 1, i + t), v1);
+      }
+    }
+    *reinterpret_cast<double2*>(out + 2 * size_t(rid)) = make_double2(v0, v1);
+  }
+  __syncwarp();
 }
 
 // Raises the non-finite flag when a new displacement pair holds a NaN or an

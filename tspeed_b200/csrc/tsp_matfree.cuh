@@ -502,12 +502,18 @@ __global__ void __launch_bounds__(MFCfg<N>::WARPS * 32, MFCfg<N>::CTAS)
     __syncwarp();
     // ---- receivers of the tile's elements: sample u^{k+1} ----
     if (t1 > t0) {
-      const int last = min(e8 + 8, ne);
-      for (int e = e8; e < last; ++e) {
-        const int r0 = rcv_ptr_at(p, e), r1 = rcv_ptr_at(p, e + 1);
-        sample_receivers<NP>(p, r0, r1, k, 0, lane,
-                             [&](int c, int i) { return rows[c * CF::ROWS * 8 + mf_at(i, e - e8)]; });
-      }
+      const int mine = rcv_ptr_at(p, min(e8 + 1 + (lane & 7), ne));
+      int end[7];  // first receiver position behind each element of the tile
+#pragma unroll
+      for (int j = 0; j < 7; ++j) end[j] = __shfl_sync(0xffffffffu, mine, j);
+      sample_receivers<NP, NP>(p, t0, t1, k, 0, lane,
+                           [&](int r) {
+                             int el = 0;
+#pragma unroll
+                             for (int j = 0; j < 7; ++j) el += r >= end[j];
+                             return el;
+                           },
+                           [&](int el, int c, int i) { return rows[c * CF::ROWS * 8 + mf_at(i, el)]; });
     }
     // ---- edge values of u^{k+1} for the next step ----
     if (q.dout != nullptr) mf_traces<N>(trc, rows, fc, e8, ne, lane, q.dout);

@@ -524,7 +524,9 @@ __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(c
           if (q < NPAIR) *reinterpret_cast<double2*>(yw + 2 * q) = un2[s];
         }
         __syncwarp();
-        sample_receivers<NP>(p, r0, r1, k, 0, lane, [&](int c, int i) { return yw[c * NP + i]; });
+        constexpr int UN = NP == 45 ? 15 : NP == 36 ? 12 : NP % 7 == 0 ? 7 : 5;
+        sample_receivers<NP, UN>(p, r0, r1, k, 0, lane, [](int) { return 0; },
+                             [&](int, int c, int i) { return yw[c * NP + i]; });
       }
       // ---- per-mesh power-iteration sums (multi-mesh groups) ----
       if (p.mode == kModePower && p.mesh_of != nullptr) {
