@@ -344,16 +344,21 @@ __global__ void __launch_bounds__(256) k_step_rows(const StepParams p) {
     for (int b = 0; b < nb; ++b) {
       const int c = col_at(p, rb + b);
       const double2* src = reinterpret_cast<const double2*>(p.x + (size_t(c) * S + sh) * R);
-      const double xs = (p.mode == kModePower) ? power_scale(p, e) : 1.0;
       for (int q = tl; q < NPAIR; q += T) {
-        double2 v = __ldg(src + q);
-        if (p.mode == kModePower) { v.x *= xs; v.y *= xs; }
+        const double2 v = __ldg(src + q);
         xt[b][2 * q] = v.x;
         xt[b][2 * q + 1] = v.y;
       }
     }
   }
   __syncwarp();
+  if (p.mode == kModePower) {
+    if (active) {
+      const double xs = power_scale(p, e);
+      for (int q = tl; q < nb * R; q += T) (&xt[0][0])[q] *= xs;  // the blocks' x lie one after the other
+    }
+    __syncwarp();
+  }
 
   AT acc[PPL][2];
 #pragma unroll
