@@ -344,3 +344,37 @@ def test_receivers_sample_their_element(N, precision, op, per_element):
     ref = np.einsum("ri,cri->rc", phi, u[:, elem])
     assert len(set(elem)) == 6
     assert rel(seis, ref) < 1e-13
+
+
+# Sizes on both sides of the lines between kernels that lie on the number of
+# triangles: the row and the ring kernel at N = 3, few-shot and batched kernels
+# at N = 6, against the matrix-free operator.
+@pytest.mark.parametrize("N,nx,ny,shots,precision", [(3, 62, 25, 1, "fp64"), (3, 47, 33, 1, "fp64"),
+                                                     (3, 74, 25, 1, "fp64"), (3, 617, 3, 1, "fp64"),
+                                                     (3, 70, 37, 1, "fp64"), (3, 72, 36, 1, "fp64"),
+                                                     (3, 100, 60, 1, "fp64"), (3, 353, 17, 1, "fp64"),
+                                                     (6, 50, 50, 33, "fp32"), (6, 51, 50, 33, "fp32")])
+def test_lines_between_kernels_on_size(N, nx, ny, shots, precision, monkeypatch):
+    monkeypatch.delenv("TSP_BATCHED_VARIANT", raising=False)
+    m = W.jittered_rect(nx, ny, 100.0 * nx, 100.0 * ny, seed=N)
+    rng = np.random.default_rng(N)
+    vp = 2500 + 1500 * rng.random(m.ne)
+    lam, mu, rho = W.lame(vp, vp / 1.8, 2000 + 500 * rng.random(m.ne))
+    x = rng.standard_normal(m.ne * (N + 1) * (N + 2))
+    out = []
+    for op, prec, S in (("matrix_free", "fp64", 1), ("explicit", precision, shots)):
+        with capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(40.0, 30.0)] * S, [(61.0, 33.0), (20.0, 55.0)],
+                                    penalty=10.0, op=op, precision=prec) as s:
+            s.set_dt(1e-5)
+            y, lmax = s.apply(x), s.estimate_lmax(10)
+            for k in range(S):
+                s.set_ricker(k, 20.0, 0.05, -1e9, 1, 20)
+                s.set_initial(k, 1e-3 * x)
+            s.first_step()
+            s.run(9)
+            out.append((y, s.u(S - 1), s.seismograms(0, 10)[S - 1], lmax))
+    a, b = out
+    tol = 1e-11 if precision == "fp64" else 1e-4
+    for i in range(3):
+        assert rel(b[i], a[i]) < tol
+    assert abs(b[3] - a[3]) < tol * a[3]

@@ -514,6 +514,16 @@ int upload_rows(tsp_handle* h, const int* row_ptr, const int* col) {
 // 90 / 97). BF16 blocks are not multiples of the 16 bytes
 // of a bulk copy.
 constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 42); }
+// FP64 2Np = 20, the smallest rows the ring kernel takes: its step lasts as
+// many rounds as teams (seven per SM) have rows, and between three and twelve
+// thousand triangles the row kernel wins where a round has just begun. us per
+// step, ring / rows, 4 receivers: 2,800 triangles 8.5 / 8.1, 3,200 10.2 / 8.1,
+// 4,000 10.2 / 10.5; 8 receivers: 3,400 10.4 / 9.5, 3,800 10.1 / 11.4, 5,000
+// 11.9 / 13.0, 5,600 14.5 / 13.2, 8,000 17.7 / 16.8, 10,000 21.6 / 20.7, 12,000
+// 25.8 / 25.5, 15,000 31.3 / 38.4.
+constexpr bool rowring_slow(int R, bool fp64, long long ne) {
+  return fp64 && R == 20 && ((ne > 3100 && ne <= 3700) || (ne > 5180 && ne <= 12000));
+}
 // Handles of a few shots use the same storage with shot tiles of 8 to 32
 // (k_step_rowshots), unless TSP_BATCHED_VARIANT asks for a batched kernel.
 // Most shots for which that is the faster one (0: any number), from 4,900
@@ -524,13 +534,18 @@ constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 42); }
 //   FP32  20: 32 36 / 50, 64 73 / 58; 30: 8 19 / 69, 32 67 / 77, 48 98 / 84;
 //         42: 24 91 / 118, 32 130 / 121; 56: 48 247 / 252, 64 337 / 258;
 //         72: 8 72 / 608, 64 502 / 686; 90: 8 104 / 796, 64 823 / 962
+// Away from that size the few-shot kernel keeps its lead (60 to 80,000
+// triangles; where any number takes it, up to 256 shots: FP64 72, S = 128,
+// 20,000 triangles 5115 / 5437, FP32 90, S = 256, 2,000 1252 / 1546), but for
+// FP32 56 with more than 32 shots: 33 at 1,000 triangles 54 / 61, 5,000 252 / 247,
+// 7,000 351 / 338, 80,000 3988 / 3707.
 constexpr bool rowshots_size(int R) { return R >= 20; }
-int rowshots_max(int R, bool fp64) {
+int rowshots_max(int R, bool fp64, long long ne) {
   switch (R) {
     case 20: return fp64 ? 48 : 32;
     case 30: return fp64 ? 0 : 32;
     case 42: return fp64 ? 48 : 24;
-    case 56: return fp64 ? 0 : 48;
+    case 56: return fp64 ? 0 : ne <= 5000 ? 48 : 32;
     case 90: return fp64 ? 48 : 0;
     default: return 0;
   }
@@ -538,8 +553,8 @@ int rowshots_max(int R, bool fp64) {
 bool uses_rowring(const tsp_handle* h) {
   if (h->op_kind != TSP_OP_EXPLICIT || h->prec == TSP_PREC_BF16) return false;
   const bool fp64 = h->prec == TSP_PREC_FP64;
-  if (h->S == 1) return rowring_size(h->R, fp64);
-  const int most = rowshots_max(h->R, fp64);
+  if (h->S == 1) return rowring_size(h->R, fp64) && !rowring_slow(h->R, fp64, h->ne);
+  const int most = rowshots_max(h->R, fp64, h->ne);
   return rowshots_size(h->R) && h->kernel_variant < 0 && (most == 0 || h->S <= most);
 }
 
