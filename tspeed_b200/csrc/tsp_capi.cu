@@ -1300,9 +1300,14 @@ int get_shots(tsp_handle* h, const double* dsrc, int ne, int shot, int n, double
 // stride of S*R) to/from a reference-layout host vector (NULL: zeros).
 int get_shot(tsp_handle* h, const double* dsrc, int ne, int shot, double* out) {
   const int R = h->R;
-  const int rc = get_shots(h, dsrc, ne, shot, 1, out);
-  if (rc != TSP_ERR_NOMEM) return rc;
-  // No room on the device: reorder on the host.
+  // Reordered on the host where that is the shorter way (the device's takes an
+  // allocation and a launch: 50 triangles N = 3, 8 KB, 47 us against 31, N = 8,
+  // 36 KB, 45 / 38; 80 KB 56 / 55; 500 triangles N = 5, 168 KB, 69 / 73), or
+  // where the device has no room for the transposed copy.
+  if (size_t(ne) * R * sizeof(double) > (size_t(96) << 10) || !h->lref_inv.empty()) {
+    const int rc = get_shots(h, dsrc, ne, shot, 1, out);
+    if (rc != TSP_ERR_NOMEM) return rc;
+  }
   std::vector<double> slice(size_t(ne) * R);
   TSP_CUDA(h, cudaMemcpy2DAsync(slice.data(), size_t(R) * sizeof(double), dsrc + size_t(shot) * R,
                                 size_t(h->S) * R * sizeof(double), size_t(R) * sizeof(double), ne,
