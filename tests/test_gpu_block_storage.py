@@ -378,3 +378,49 @@ def test_lines_between_kernels_on_size(N, nx, ny, shots, precision, monkeypatch)
     for i in range(3):
         assert rel(b[i], a[i]) < tol
     assert abs(b[3] - a[3]) < tol * a[3]
+
+
+@pytest.mark.parametrize("N", range(1, 9))
+def test_matrix_free_with_little_device_memory(N):
+    """Where the edge values of the matrix-free tiles would take more than a
+    quarter of the free memory, the handle steps without them."""
+    rt = ctypes.CDLL("libcudart.so.12")
+    rt.cudaMemGetInfo.argtypes = [ctypes.POINTER(ctypes.c_size_t)] * 2
+    m = W.jittered_rect(200, 180, 2000.0, 1800.0, seed=N)
+    kept = m.ne * (46 + 24 * (N + 1)) * 8  # 54 MB (N = 1) to 151 MB
+    rng = np.random.default_rng(N)
+    vp = 2500 + 1500 * rng.random(m.ne)
+    lam, mu, rho = W.lame(vp, vp / 1.8, 2000 + 500 * rng.random(m.ne))
+    x = rng.standard_normal(m.ne * (N + 1) * (N + 2))
+    out, ballast = [], []
+    try:
+        for little in (False, True):
+            if little:
+                capi.release_cached_memory(0)
+                room, total, p = ctypes.c_size_t(), ctypes.c_size_t(), ctypes.c_void_p()
+                while True:
+                    assert rt.cudaMemGetInfo(ctypes.byref(room), ctypes.byref(total)) == 0
+                    spare = room.value - 3 * kept
+                    if spare < (16 << 20) or rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(min(spare, 1 << 30))) != 0:
+                        break
+                    ballast.append(ctypes.c_void_p(p.value))
+                rt.cudaGetLastError()
+            with capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(1010.0, 905.0)], [(1031.0, 933.0), (20.0, 55.0)],
+                                        penalty=10.0, op="matrix_free") as s:
+                y, lmax = s.apply(x), s.estimate_lmax(6)
+                s.set_dt(1e-5)
+                s.set_ricker(0, 20.0, 0.05, -1e9, 1, 20)
+                s.set_initial(0, 1e-3 * x)
+                s.enable_energy(True)
+                s.first_step()
+                s.run(9)
+                out.append((y, s.u(), s.seismograms(0, 10), s.energy(1, 9), lmax))
+    finally:
+        for p in ballast:
+            rt.cudaFree(p)
+    a, b = out
+    assert not np.array_equal(a[0], b[0])  # another kernel
+    assert rel(b[0], a[0]) < 1e-13
+    assert abs(b[4] - a[4]) < 1e-12 * a[4]
+    for i in (1, 2, 3):
+        assert rel(b[i], a[i]) < 1e-11

@@ -27,6 +27,7 @@
 #include "tsp_simt32.cuh"
 #include "tsp_rowring.cuh"
 #include "tsp_matfree.cuh"
+#include "tsp_matfree_lean.cuh"
 #include "tsp_rowshots.cuh"
 
 namespace {
@@ -70,6 +71,7 @@ struct tsp_handle {
   // matrix-free operator: reference tables, per-element data, and the edge
   // values of each state level (like d_U, d_D[i] belongs to d_U[i])
   tsp::MatFreeParams mf = {};
+  tsp::MatFreeLeanParams mf_lean = {};  // tables != null: the lean kernel steps this handle
   double* d_D[2] = {nullptr, nullptr};
   // multi-mesh group (set by tsp_batch_create; null for ordinary handles)
   double* d_dt_elem = nullptr;
@@ -792,7 +794,40 @@ int launch_matfree_N(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   return TSP_OK;
 }
 
+template <int N>
+int launch_matfree_lean_N(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
+  typedef tsp::MFLeanCfg<N> CF;
+  const size_t smem = CF::smem_bytes();
+  static unsigned long long configured = 0;
+  const unsigned long long bit = 1ull << (h->device & 63);
+  if (!(configured & bit)) {
+    cudaError_t e = cudaFuncSetAttribute(tsp::k_step_matfree_lean<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return fail(h, TSP_ERR_CUDA, std::string("lean matrix-free kernel smem: ") + cudaGetErrorString(e));
+    configured |= bit;
+  }
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tsp::k_step_matfree_lean<N>, CF::WARPS * 32, smem);
+  const long long want = (h->ne + CF::WARPS - 1) / CF::WARPS;
+  const unsigned grid = unsigned(std::min<long long>(want, (long long)std::max(per_sm, 1) * h->num_sms));
+  tsp::k_step_matfree_lean<N><<<grid, CF::WARPS * 32, smem, st>>>(p, h->mf_lean);
+  return TSP_OK;
+}
+
+int launch_matfree_lean(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
+  switch (h->N) {
+    case 1: return launch_matfree_lean_N<1>(h, p, st);
+    case 2: return launch_matfree_lean_N<2>(h, p, st);
+    case 3: return launch_matfree_lean_N<3>(h, p, st);
+    case 4: return launch_matfree_lean_N<4>(h, p, st);
+    case 5: return launch_matfree_lean_N<5>(h, p, st);
+    case 6: return launch_matfree_lean_N<6>(h, p, st);
+    case 7: return launch_matfree_lean_N<7>(h, p, st);
+    default: return launch_matfree_lean_N<8>(h, p, st);
+  }
+}
+
 int launch_matfree(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
+  if (h->mf_lean.tables) return launch_matfree_lean(h, p, st);
   switch (h->N) {
     case 1: return launch_matfree_N<1>(h, p, st);
     case 2: return launch_matfree_N<2>(h, p, st);
@@ -807,6 +842,7 @@ int launch_matfree(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
 }
 
 int refresh_matfree(tsp_handle* h, int i) {
+  if (h->mf_lean.tables) return TSP_OK;
   switch (h->N) {
     case 1: return launch_matfree_traces<1>(h, h->d_U[i], i, h->stream);
     case 2: return launch_matfree_traces<2>(h, h->d_U[i], i, h->stream);
@@ -850,6 +886,52 @@ std::vector<double> matfree_tables(int N, const tsp::RefTables& T) {
           pk.push_back(r < RQ && j < Np ? edge(part, r, j) : 0.0);
         }
   return pk;
+}
+
+// Packed tables of MFLeanCfg<N>: KT[ab][j][i], TRT[l][j][r], TR[l][r][i] (r < Q:
+// basis, Q <= r < 3Q: gradient a = r / Q - 1), w1.
+std::vector<double> matfree_lean_tables(const tsp::RefTables& T) {
+  const int Np = T.Np, Q = T.Q, Q3 = 3 * Q;
+  const size_t P2 = size_t(Np) * Np;
+  std::vector<double> pk(4 * P2 + 2 * size_t(3) * Np * Q3 + Q);
+  double* KT = pk.data();
+  double* TRT = KT + 4 * P2;
+  double* TR = TRT + size_t(3) * Np * Q3;
+  for (int ab = 0; ab < 4; ++ab)
+    for (int i = 0; i < Np; ++i)
+      for (int j = 0; j < Np; ++j) KT[(size_t(ab) * Np + j) * Np + i] = T.K[ab * P2 + size_t(i) * Np + j];
+  for (int l = 0; l < 3; ++l)
+    for (int r = 0; r < Q3; ++r)
+      for (int j = 0; j < Np; ++j) {
+        const int kq = r % Q, part = r / Q;
+        const double v = part == 0 ? T.Be[(size_t(l) * Q + kq) * Np + j]
+                                   : T.Ge[((size_t(l) * 2 + (part - 1)) * Q + kq) * Np + j];
+        TRT[(size_t(l) * Np + j) * Q3 + r] = v;
+        TR[(size_t(l) * Q3 + r) * Np + j] = v;
+      }
+  std::copy(T.w1.begin(), T.w1.begin() + Q, TR + size_t(3) * Q3 * Np);
+  return pk;
+}
+
+// Whether a matrix-free handle of ne elements does without the tiled kernel's
+// edge values and records: where these would take more than a quarter of the
+// device memory that is free now (the pool's cached memory counts as free), so
+// that meshes up to the size that the lean form fits stay possible, with room
+// for the vectors that later calls allocate.
+bool matfree_lean(tsp_handle* h, int Q) {
+  const size_t kept = size_t(h->ne) * (46 + 2 * 3 * size_t(Q) * 4) * sizeof(double);
+  size_t room = 0, total = 0;
+  if (cudaMemGetInfo(&room, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  cudaMemPool_t pool = nullptr;
+  uint64_t reserved = 0, used = 0;
+  if (device_pool(h->device, &pool) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+    room += size_t(reserved - used);
+  return kept > room / 4;
 }
 
 template <int R, int ST, int TR>
@@ -1572,6 +1654,16 @@ int tsp_create(const tsp_problem* P, tsp_handle** out) {
       (rc = upload(h, &d_Ds, T.Ds.data(), T.Ds.size())) || (rc = upload(h, &d_Dx, T.Dx.data(), T.Dx.size())))
     return create_error_from(h, rc);
   h->bpitch = h->bref.empty() ? block_pitch(h->R, h->S) : h->R;
+  if (h->op_kind == TSP_OP_MATRIX_FREE && matfree_lean(h, T.Q)) {
+    const std::vector<double> pk = matfree_lean_tables(T);
+    double* d_tab = nullptr;
+    if ((rc = upload(h, &d_tab, pk.data(), pk.size()))) return create_error_from(h, rc);
+    h->mf_lean = {d_tab, d_invJ, d_detJ, d_lam, d_mu, d_elen, d_enrm, d_neigh, d_nedge, P->penalty * h->N * h->N};
+    for (void* q : {(void*)d_bface, (void*)d_K, (void*)d_Ws, (void*)d_Wx, (void*)d_Ds, (void*)d_Dx}) dfree(h, q);
+    if ((rc = finish_create(h))) return create_error_from(h, rc);
+    *out = h;
+    return TSP_OK;
+  }
   if (h->op_kind == TSP_OP_MATRIX_FREE) {
     const std::vector<double> pk = matfree_tables(P->N, T);
     double *d_tab = nullptr, *d_alpha = nullptr, *d_face = nullptr;
