@@ -72,3 +72,28 @@ def test_estimate_between_queued_steps_leaves_the_run_alone(N, nx, ny, op, preci
     assert all(np.any(u) for u in out[0][:2])
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+# Groups on both sides of the sizes between which matrix-free groups of a batch
+# of three and more degrees are stepped by the lean kernel.
+@pytest.mark.parametrize("nx,ny", [(10, 10), (17, 6), (25, 20), (21, 24)])
+def test_matrix_free_batch_of_three_degrees(nx, ny):
+    probs = []
+    for N in (2, 4, 7):
+        m = W.jittered_rect(nx, ny, 100.0 * nx, 100.0 * ny, seed=N)
+        lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+        probs.append(W.Problem(str(N), m, N, lam, mu, rho, [W.Source(51.0 * nx, 47.0 * ny, 200.0, 1e-3, -1e9, 1)],
+                               [(52.0 * nx, 49.0 * ny), (50.0, 60.0)], 30))
+    with capi.Batch(probs, op="matrix_free") as b:
+        b.set_dt(np.full(3, 1e-4))
+        b.set_ricker(30)
+        b.first_step()
+        b.run(29)
+        out = [(b.u(i), b.seismograms(i, 0, 30)) for i in range(3)]
+    for p, (u, seis) in zip(probs, out):
+        with capi.Simulation.from_problem(p, op="matrix_free") as s:
+            s.set_dt(1e-4)
+            s.set_ricker(0, 200.0, 1e-3, -1e9, 1, 30)
+            s.first_step()
+            s.run(29)
+            assert rel(u, s.u()) < 1e-12 and rel(seis, s.seismograms(0, 30)[0]) < 1e-12

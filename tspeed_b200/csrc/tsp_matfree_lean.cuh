@@ -11,7 +11,8 @@
 // It serves where the tiled kernel's edge values and records do not fit: 16
 // doubles and 24 bytes of geometry per element instead of 46 doubles and two
 // levels of 12 (N + 1) (N = 6 with both state levels 1.1 KB per element instead
-// of 2.6).
+// of 2.6); and small groups of batches of several degrees, whose unrolled tiled
+// kernels would evict one another from the instruction caches.
 //   volume   y^m += |detJ| sum_ab K^{ab} (sum_n alpha^{mn}_ab x^n)
 //   face l   with J^n(k) = u_e^n(k) - u_nb^n(Q-1-k) (jump at edge point k),
 //            T_e^m(k) = sum_{n,a} beta^{nm}_a(e) g_e^n_a(k) (traction of u_e),
