@@ -75,27 +75,31 @@ def captured_traffic(kernel, ne, nshots):
 
 # Batched FP32 step kernels by variant (tsp_get_kernel_variant), for 2Np = 42.
 KERNELS = {0: "k_step_batched32k<42>", 1: "k_step_batched32p<42,64,4>", 2: "k_step_batched32<42>",
-           4: "k_step_batched_fx<42>", 7: "k_step_batched32w<42,3,3,2,1,6>", 8: "k_step_batched32w<42,4,2,2,1,3>",
-           14: "k_step_rowshots<42>"}
+           4: "k_step_batched_fx<42>", 7: "k_step_batched32w<42,3,3,2,1,6>", 8: "k_step_batched32w<42,4,2,2,1,3>"}
 
 
-def ring_kernel(R, precision):
-    """Whether a single-shot explicit handle runs k_step_rowring (else k_step_rows)."""
-    return R >= {"fp64": 20, "fp32": 42}.get(precision, 1 << 30)
+def step_kernel(sim, precision):
+    """Kernel that steps an explicit handle; fewer stored blocks than the
+    pattern's: the single-shot ring kernel or the few-shot kernel."""
+    R, v = 2 * sim.Np, sim.kernel_variant
+    if sim.stored_blocks < sim.nnzb:
+        return f"k_step_{'rowring' if sim.nshots == 1 else 'rowshots'}<{R},{'double' if precision == 'fp64' else 'float'}>"
+    if sim.nshots == 1:
+        return f"k_step_rows<{R},{ {'fp64': 'double', 'fp32': 'float'}.get(precision, 'bf16')}>"
+    return (KERNELS.get(v, "batched") if precision == "fp32" else
+            D64_KERNELS.get(v, "batched") if precision == "fp64" else "k_step_batched<42>")
 
 
-def bytes_per_step(ne, Np, nnzb, nshots, precision):
-    """Algorithmic HBM bytes of one step: every stored block once, the state
+def bytes_per_step(ne, Np, stored, nshots, precision):
+    """Algorithmic HBM bytes of one step: every stored block once (one per face
+    where the operator is stored symmetrically, both rows use it), the state
     read (u^k, u^{k-1}) and written (u^{k+1}) once per shot, minv once. The
     tensor-core form ("fx") stores each operator entry as three BF16
-    fixed-point slices (6 bytes). Single-shot handles with larger blocks store
-    one block per face (the operator is symmetric; both rows use it)."""
+    fixed-point slices (6 bytes)."""
     R = 2 * Np
-    if nshots == 1 and ring_kernel(R, precision):
-        nnzb = ne + (nnzb - ne) // 2
     bblk = {"fp64": 8, "fp32": 4, "bf16": 2, "fx": 6}[precision]
-    extra = nnzb * 4 if precision == "bf16" else 0
-    return nnzb * R * R * bblk + extra + nshots * 2 * ne * Np * 24 + ne * 8
+    extra = stored * 4 if precision == "bf16" else 0
+    return stored * R * R * bblk + extra + nshots * 2 * ne * Np * 24 + ne * 8
 
 
 class ClockSampler:
@@ -476,10 +480,10 @@ def single_shot_forms(args):
             s.run_timed(K)
             ms = s.run_timed(K)
             seis[form] = s.seismograms(0, total)
-            nnzb = s.nnzb
+            stored = s.stored_blocks
         d = {"ms_per_step": ms / K, "value": prob.dofs_per_shot * K / (ms / 1e3)}
         if op == "explicit":
-            algo = bytes_per_step(prob.mesh.ne, prob.Np, nnzb, 1, prec)
+            algo = bytes_per_step(prob.mesh.ne, prob.Np, stored, 1, prec)
             d["roofline_frac"] = algo / (ms / K / 1e3) / 1e9 / hbm
             d["algorithmic_bytes_per_step"] = algo
         out["forms"][form] = d
@@ -574,12 +578,9 @@ def main():
     ms_step = ms / K
     hbm, peak_kind = peaks()
     form = "fx" if variant == 4 else args.precision
-    algo = bytes_per_step(prob.mesh.ne, prob.Np, sim.nnzb, prob.nshots, form)
+    algo = bytes_per_step(prob.mesh.ne, prob.Np, sim.stored_blocks, prob.nshots, form)
     achieved = algo / (ms_step / 1e3) / 1e9
-    kernel = (KERNELS.get(variant, "batched") if variant is not None else
-              f"k_step_{'rowring' if ring_kernel(2 * prob.Np, args.precision) else 'rows'}<{2 * prob.Np}>"
-              if prob.nshots == 1 else
-              D64_KERNELS.get(variant64, "batched") if args.precision == "fp64" else "k_step_batched<42>")
+    kernel = step_kernel(sim, args.precision)
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": Wm,
             "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": ("bf16x3 fixed-point operator, f64 state" if form == "fx" else
@@ -587,11 +588,7 @@ def main():
                       "bf16 operator, f64 state" if args.precision == "bf16" else "f64"), "data": "synthetic",
             "config": config_dict(args, prob), "dt": dt, "lmax": lmax,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                         "traffic": (captured_traffic(kernel, prob.mesh.ne, prob.nshots)
-                                     if variant is not None else
-                                     captured_traffic("k_step_rowring<42,double>", prob.mesh.ne, prob.nshots)
-                                     if prob.nshots == 1 and args.precision == "fp64" else None)
-                         if prob.N == 5 else None,
+                         "traffic": captured_traffic(kernel, prob.mesh.ne, prob.nshots) if prob.N == 5 else None,
                          "traffic_source": "ncu capture (profiles/traffic.json) scaled by element rows",
                          "kernel": kernel, "kernel_variant": variant,
                          "peak_source": peak_kind,
@@ -619,9 +616,9 @@ def main():
             s1.run(Wm)
             s1.run_timed(K)
             ms1 = s1.run_timed(K)
-            nnzb1 = s1.nnzb
+            stored1 = s1.stored_blocks
         v1 = p1.dofs_per_shot * K / (ms1 / 1e3)
-        a1 = bytes_per_step(p1.mesh.ne, p1.Np, nnzb1, 1, "fp64") / (ms1 / K / 1e3) / 1e9
+        a1 = bytes_per_step(p1.mesh.ne, p1.Np, stored1, 1, "fp64") / (ms1 / K / 1e3) / 1e9
         line["plain_fp64_single_shot"] = {"value": v1, "unit": UNIT, "ms_per_step": ms1 / K,
                                           "roofline_frac": a1 / hbm, "achieved_gbs": a1}
         line["speedup_vs_plain_fp64"] = value / v1
@@ -632,14 +629,15 @@ def main():
             s1f.run(Wm)
             s1f.run_timed(K)
             ms1f = s1f.run_timed(K)
-        a1f = bytes_per_step(p1.mesh.ne, p1.Np, nnzb1, 1, "fp32") / (ms1f / K / 1e3) / 1e9
+            stored1f = s1f.stored_blocks
+        a1f = bytes_per_step(p1.mesh.ne, p1.Np, stored1f, 1, "fp32") / (ms1f / K / 1e3) / 1e9
         line["plain_fp32_operator_single_shot"] = {"value": p1.dofs_per_shot * K / (ms1f / 1e3), "unit": UNIT,
                                                    "ms_per_step": ms1f / K, "roofline_frac": a1f / hbm,
                                                    "achieved_gbs": a1f, "speedup_vs_plain_fp64": ms1 / ms1f}
         # Mixed precision for all shots: FP32 operator, autotuned batched kernel.
         if prob.nshots > 1 and args.precision == "fp64":
             with capi.Simulation.from_problem(prob, precision="fp32") as s32:
-                v32var = s32.kernel_variant
+                v32var, k32 = s32.kernel_variant, step_kernel(s32, "fp32")
                 prepare(s32, prob, dt, K + Wm + 2)
                 s32.first_step()
                 s32.run(Wm)
@@ -648,11 +646,11 @@ def main():
             v32 = prob.nshots * dofs * K / (ms32 / 1e3)
             line["batched_fp32_operator"] = {"value": v32, "unit": UNIT, "ms_per_step": ms32 / K,
                                              "speedup_vs_plain_fp64": v32 / v1,
-                                             "kernel": KERNELS.get(v32var, "batched"), "kernel_variant": v32var}
+                                             "kernel": k32, "kernel_variant": v32var}
         # Exact FP64 for all shots: the FP64 tensor-core batched step.
         if prob.nshots > 1 and args.precision != "fp64":
             with capi.Simulation.from_problem(prob, precision="fp64") as s64:
-                v64var = s64.kernel_variant
+                k64 = step_kernel(s64, "fp64")
                 prepare(s64, prob, dt, K + Wm + 2)
                 s64.first_step()
                 s64.run(Wm)
@@ -663,7 +661,7 @@ def main():
             line["batched_fp64"] = {"value": v64, "unit": UNIT, "ms_per_step": ms64 / K,
                                     "speedup_vs_plain_fp64": v64 / v1, "seismogram_err": "exact FP64",
                                     "roofline": fp64_tensor_roofline(nnzb64, prob.Np, prob.nshots, ms64 / K,
-                                                                     D64_KERNELS.get(v64var, "batched"))}
+                                                                     k64)}
         # Accuracy of the measured form over the full step count against FP64
         # computed by the CUDA-core FP64 kernel (TSP_BATCHED_VARIANT=2): for the
         # FP64 tensor-core form this is the difference of two FP64 summation

@@ -186,6 +186,10 @@ const char* tsp_last_error(const tsp_handle* h);
 
 /* Problem sizes: ne, Np, nshots, nrcv, nnzb (NULL pointers are skipped). */
 int tsp_get_sizes(const tsp_handle* h, int32_t* ne, int32_t* Np, int32_t* nshots, int32_t* nrcv, int64_t* nnzb);
+/* Blocks held on the device: nnzb, fewer where a symmetric operator is stored
+ * once per face (the single-shot ring kernel and the few-shot kernel), 0 for
+ * the matrix-free operator. */
+int tsp_get_stored_blocks(const tsp_handle* h, int64_t* stored);
 
 /* TimeAdvance::set_dt (TimeAdvance.hpp:153). */
 int tsp_set_dt(tsp_handle* h, double dt);
@@ -243,7 +247,8 @@ int tsp_run_timed(tsp_handle* h, int64_t nsteps, double* ms);
  * latency, 9 and 10 the epilogue in update warps, 3 single-role DMMA kernel,
  * 2 CUDA-core kernel. Handles of a few shots (how few depends on the degree)
  * take the DMMA kernel with shot tiles of 8 to 32 on symmetric block storage
- * without a trial: reported as 5 for an FP64 operator, 14 for an FP32 one.
+ * without a trial: reported as 5 for an FP64 operator (as the batched kernel 5;
+ * tsp_get_stored_blocks tells them apart), 14 for an FP32 one.
  * No counterpart in the reference (its step is a single CPU path). */
 int tsp_get_kernel_variant(const tsp_handle* h, int32_t* variant);
 

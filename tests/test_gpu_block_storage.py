@@ -424,3 +424,27 @@ def test_matrix_free_with_little_device_memory(N):
     assert abs(b[4] - a[4]) < 1e-12 * a[4]
     for i in (1, 2, 3):
         assert rel(b[i], a[i]) < 1e-11
+
+
+def test_reported_kernels(monkeypatch):
+    """A forced number that names no FP32 batched kernel is reported as the
+    kernel that runs; stored blocks tell symmetric storage from full."""
+    m = W.jittered_rect(8, 5, 800.0, 500.0, seed=2)
+    lam, mu, rho = W.lame(np.full(m.ne, 3000.0), np.full(m.ne, 1700.0), np.full(m.ne, 2300.0))
+    nnzb = m.ne + 2 * ((3 * m.ne - 2 * (8 + 5)) // 2)
+
+    def handle(N, shots, precision, op="explicit"):
+        return capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(310.0 + k, 240.0) for k in range(shots)], [],
+                                      penalty=10.0, precision=precision, op=op)
+    for N, shown in ((4, 1), (6, 1), (7, 2)):
+        monkeypatch.setenv("TSP_BATCHED_VARIANT", "14")
+        with handle(N, 3, "fp32") as s:
+            assert s.kernel_variant == shown and s.stored_blocks == s.nnzb == nnzb
+    monkeypatch.delenv("TSP_BATCHED_VARIANT")
+    half = m.ne + (nnzb - m.ne) // 2
+    for N, shots, precision, op, stored in ((5, 1, "fp64", "explicit", half), (5, 3, "fp64", "explicit", half),
+                                            (5, 3, "fp32", "explicit", half), (5, 64, "fp32", "explicit", nnzb),
+                                            (2, 1, "fp64", "explicit", nnzb), (5, 1, "bf16", "explicit", nnzb),
+                                            (5, 1, "fp64", "matrix_free", 0)):
+        with handle(N, shots, precision, op) as s:
+            assert s.nnzb == nnzb and s.stored_blocks == stored

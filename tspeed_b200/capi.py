@@ -103,6 +103,7 @@ SIGNATURES = {
     "tsp_set_initial_values": (C.c_int, [C.c_void_p, C.c_int32, _dp, _dp]),
     "tsp_release_cached_memory": (C.c_int, [C.c_int32]),
     "tsp_fp64_tensor_peak": (C.c_int, [C.c_int32, _dp]),
+    "tsp_get_stored_blocks": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64)]),
     "tsp_selftest_bounded_wait": (C.c_int, [C.c_int32, _ip, _ip]),
     "tsp_selftest_set_timeout": (C.c_int, [C.c_void_p, C.c_int32]),
     "tsp_selftest_batch_set_timeout": (C.c_int, [C.c_void_p, C.c_int32]),
@@ -368,6 +369,14 @@ class Simulation:
         return k.value, t.value
 
     @property
+    def stored_blocks(self) -> int:
+        """Blocks held on the device: nnzb, fewer on symmetric storage, 0
+        matrix-free."""
+        n = C.c_int64()
+        _check(lib().tsp_get_stored_blocks(self._h, C.byref(n)), self._h)
+        return n.value
+
+    @property
     def kernel_variant(self) -> int:
         """Batched-step kernel chosen by the autotuner (or TSP_BATCHED_VARIANT):
         FP32: 7/8 warp-specialised CUDA-core kernels with bulk-copy rings,
@@ -375,7 +384,8 @@ class Simulation:
         with several shots: 5 and 6 warp-specialised FP64 tensor-core kernels
         (two groups of 8 consumer warps / one group of 16), 3 single-role
         one, 2 CUDA-core kernel. Few shots: 5 (FP64) or 14 (FP32), the
-        few-shot kernel on symmetric storage (no trial)."""
+        few-shot kernel on symmetric storage (no trial; fewer stored_blocks
+        than nnzb)."""
         v = C.c_int32()
         _check(lib().tsp_get_kernel_variant(self._h, C.byref(v)), self._h)
         return v.value

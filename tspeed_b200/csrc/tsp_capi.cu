@@ -401,6 +401,10 @@ int autotune(tsp_handle* h) {
     }
   } else if (h->kernel_variant >= 0 || !h->shadow) {
     if (h->kernel_variant < 0) h->kernel_variant = 0;
+    // A number that names no FP32 batched kernel runs the pipelined one, or the
+    // plain one where that is not built (see launch_R): reported as such.
+    const int v = h->kernel_variant;
+    if (h->shadow && v != 0 && v != 1 && v != 2 && v != 4 && v != 7 && v != 8) h->kernel_variant = h->R <= 56 ? 1 : 2;
     return TSP_OK;
   }
   const auto key = std::make_tuple(h->device, h->prec, h->R, h->S, h->ne);
@@ -1949,6 +1953,12 @@ int tsp_get_sizes(const tsp_handle* h, int32_t* ne, int32_t* Np, int32_t* nshots
   if (nshots) *nshots = h->S;
   if (nrcv) *nrcv = h->nrcv;
   if (nnzb) *nnzb = h->nnzb;
+  return TSP_OK;
+}
+
+int tsp_get_stored_blocks(const tsp_handle* h, int64_t* stored) {
+  if (!h || !stored) return TSP_ERR_ARG;
+  *stored = h->op_kind == TSP_OP_MATRIX_FREE ? 0 : h->nstored;
   return TSP_OK;
 }
 
