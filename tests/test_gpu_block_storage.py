@@ -448,3 +448,32 @@ def test_reported_kernels(monkeypatch):
                                             (5, 1, "fp64", "matrix_free", 0)):
         with handle(N, shots, precision, op) as s:
             assert s.nnzb == nnzb and s.stored_blocks == stored
+
+
+# FP32 blocks of the few-shot kernel are widened and multiply the FP64 state:
+# against the oracle on the rounded blocks only the order of FP64 sums differs
+# (bounds as for FP64 blocks above).
+@pytest.mark.parametrize("N,S", [(3, 2), (3, 32), (4, 9), (4, 24), (5, 16), (5, 24), (6, 25), (6, 48), (7, 32), (7, 70),
+                                 (8, 3), (8, 24)])
+def test_few_shots_of_fp32_blocks_sum_in_fp64(N, S, monkeypatch):
+    monkeypatch.delenv("TSP_BATCHED_VARIANT", raising=False)
+    ne, Np = 11, (N + 1) * (N + 2) // 2
+    row_ptr, col, blocks, minv = random_operator(ne, N, N + S, True)
+    rng = np.random.default_rng(S)
+    u0 = rng.standard_normal((S, 2 * ne * Np))
+    phi = rng.standard_normal((S, Np))
+    F = rng.standard_normal((S, 3, 2))
+    with capi.Simulation.from_blocks(row_ptr, col, blocks, minv, [5] * S, phi, [4], phi[:1], precision="fp32") as s:
+        assert s.stored_blocks < s.nnzb
+        s.set_dt(0.01)
+        for k in range(S):
+            s.set_force_table(k, F[k])
+            s.set_initial(k, u0[k])
+        s.first_step()
+        s.run(2)
+        u, seis = s.u_all(), s.seismograms(0, 3)
+    rounded = blocks.astype(np.float32).astype(np.float64)
+    for k in range(S):
+        ur, sr, _ = O.leapfrog(row_ptr, col, rounded, minv, ne, Np, 0.01, 3, 5, phi[k], F[k], [4], phi[:1], u0[k])
+        assert rel(u[k], ur) < 1e-12
+        assert rel(seis[k], sr) < 1e-12
