@@ -77,7 +77,6 @@ struct tsp_handle {
   double* d_dt_elem = nullptr;
   int* d_src_of = nullptr;
   int* d_mesh_of = nullptr;
-  double* d_xscale_mesh = nullptr;
   int nmesh = 0;
   // state
   double* d_U[2] = {nullptr, nullptr};
@@ -758,10 +757,10 @@ int launch_matfree_traces(tsp_handle* h, const double* x, int to, cudaStream_t s
   return TSP_OK;
 }
 
-// A step reads the edge values of its level and writes those of the new one.
-// kModeFirst computes its level's first. A single product (kModeApply,
-// kModePower) computes its vector's into the buffer that the next step will
-// write: the current level's stay valid.
+// A step reads the edge values of its level (those of u^0 are computed by
+// refresh_matfree before the first) and writes those of the new one. A single
+// product (kModeApply, kModePower) computes its vector's into the buffer that
+// the next step will write: the current level's stay valid.
 template <int N>
 int launch_matfree_N(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   typedef tsp::MFCfg<N> CF;
@@ -777,7 +776,7 @@ int launch_matfree_N(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   tsp::MatFreeParams q = h->mf;
   const bool stepping = p.mode == tsp::kModeStep || p.mode == tsp::kModeFirst;
   const int from = stepping ? (p.x == h->d_U[0] ? 0 : 1) : 1 - h->cur;
-  if (p.mode != tsp::kModeStep) {
+  if (!stepping) {
     int rc = launch_matfree_traces<N>(h, p.x, from, st);
     if (rc) return rc;
   }
@@ -1253,7 +1252,6 @@ int launch_step(tsp_handle* h, int mode, const double* x, const double* uprev, d
   p.dt_elem = h->d_dt_elem;
   p.src_of = h->d_src_of;
   p.mesh_of = (mode == tsp::kModePower) ? h->d_mesh_of : nullptr;
-  p.xscale_mesh = (mode == tsp::kModePower) ? h->d_xscale_mesh : nullptr;
   if (h->op_kind == TSP_OP_MATRIX_FREE) return launch_matfree(h, p, st);
   switch (h->R) {
     case 6: return launch_R<6>(h, p, st);
@@ -3055,7 +3053,7 @@ int tsp_batch_create(const tsp_problem* meshes, int32_t nmesh, tsp_batch** out) 
     }
     b->groups.push_back(h);
     b->group_meshes.push_back(ms);
-    // Per-mesh sources and receivers, mesh ids, per-mesh power scales.
+    // Per-mesh sources and receivers, mesh ids.
     h->nmesh = int(ms.size());
     h->src_elem.assign(1, -1);
     h->src_phi = src_phi;  // [nmesh][Np], row = source index
@@ -3071,11 +3069,10 @@ int tsp_batch_create(const tsp_problem* meshes, int32_t nmesh, tsp_batch** out) 
     h->d_rcv_id = nullptr;
     h->d_rcv_phi = nullptr;
     h->d_rcv_phi_t = nullptr;
-    std::vector<double> ones(ms.size(), 1.0);
     if ((rc = upload(h, &h->d_src_phi, src_phi.data(), src_phi.size())) ||
         (rc = upload(h, &h->d_src_of, src_of.data(), src_of.size())) ||
         (rc = upload(h, &h->d_mesh_of, mesh_of.data(), mesh_of.size())) ||
-        (rc = upload(h, &h->d_xscale_mesh, ones.data(), ones.size())) || (rc = build_receiver_csr(h)) ||
+        (rc = build_receiver_csr(h)) ||
         (rc = alloc_seis(h, h->seis_cap)) || (rc = dalloc(h, &h->d_dt_elem, size_t(ebase)))) {
       const std::string msg = h->err;
       tsp_batch_destroy(b);

@@ -75,7 +75,6 @@ struct StepParams {
   const double* dt_elem;      // per-element time step (the element's mesh's dt)
   const int* src_of;          // per-element source index into src_phi/F, -1 if none
   const int* mesh_of;         // per-element mesh id (power iteration per mesh)
-  const double* xscale_mesh;  // per-mesh power-iteration scale
   // Tensor-core fixed-point path: slice images of the state (per element and
   // 64-shot tile) and of the operator (per block), with the shared binary
   // exponents of their rows (per shot of a tile, per block row).
@@ -157,7 +156,7 @@ __device__ __forceinline__ double power_scale(const StepParams& p, int e) {
     const double s = p.acc_prev[3 * size_t(p.mesh_of != nullptr ? p.mesh_of[e] : 0) + 2];
     return s > 0 ? 1.0 / sqrt(s) : 1.0;
   }
-  return p.xscale_mesh ? p.xscale_mesh[p.mesh_of[e]] : p.xscale;
+  return p.xscale;
 }
 
 // Receivers [q0, q1) sampled by a whole warp; elem(q) names the element of

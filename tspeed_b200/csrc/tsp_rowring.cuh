@@ -88,14 +88,17 @@ struct RowRingCfg {
   static constexpr int DEPTH = NS >= NCH ? NS / NCH : 1;
   static constexpr int LAP = NS >= NCH ? 1 : NCH / NS;  // uses of a slot per block
   static_assert(NS >= NCH ? NS % NCH == 0 : NCH % NS == 0, "a chunk's slot is known at compile time");
+  // FP32: sums in column order (see ORD in the kernel): no lane groups over the
+  // columns, no parts of a column, no staggering.
+  static constexpr bool ORD = !F64;
   static constexpr int PPL = (NPAIR + 31) / 32;              // row pairs per lane
-  static constexpr int G = NPAIR <= 16 ? 32 / NPAIR : 1;     // lane groups over columns
+  static constexpr int G = !ORD && NPAIR <= 16 ? 32 / NPAIR : 1;  // lane groups over columns
   static constexpr int CPL = (NC + 31) / 32;                 // transposed: columns per lane
   static_assert(NC % CPL == 0, "columns split evenly over the lanes");
   static constexpr int LC = NC / CPL;                        // transposed: lanes per row part
-  static constexpr int PT = 32 / LC < 3 ? 32 / LC : (NPAIR % 3 == 0 ? 3 : 2);  // transposed: lanes per column
+  static constexpr int PT = ORD ? 1 : 32 / LC < 3 ? 32 / LC : (NPAIR % 3 == 0 ? 3 : 2);  // transposed: lanes per column
   static constexpr int JN = (NPAIR + PT - 1) / PT;           // row pairs per lane, transposed
-  static constexpr bool ROT = NPAIR % 2 == 0;                // stagger columns over the banks
+  static constexpr bool ROT = !ORD && NPAIR % 2 == 0;        // stagger columns over the banks
   static_assert(!ROT || NPAIR % PT == 0, "staggered parts are even");
   static constexpr int XB = ((R * int(sizeof(typename AccOf<BT>::type)) + 15) / 16) * 16;
   static constexpr int PER = NS * CB + XB;                   // one warp: ring and x of its block
@@ -157,9 +160,8 @@ template <int R, typename BT>
 __global__ void __launch_bounds__(128, RowRingCfg<R, BT>::CTAS) k_step_rowring(const StepParams p, int* err_flag) {
   typedef RowRingCfg<R, BT> CF;
   typedef typename AccOf<BT>::type AT;
-  constexpr bool ORD = !CF::F64;
-  constexpr int G = ORD ? 1 : CF::G, PT = ORD ? 1 : CF::PT, JN = ORD ? CF::NPAIR : CF::JN;
-  constexpr bool ROT = CF::ROT && !ORD;
+  constexpr bool ORD = CF::ORD, ROT = CF::ROT;
+  constexpr int G = CF::G, PT = CF::PT, JN = CF::JN;
   constexpr int NP = R / 2, NPAIR = CF::NPAIR, NC = CF::NC, NCH = CF::NCH, NS = CF::NS, PPL = CF::PPL, W = CF::W;
   constexpr int DEPTH = CF::DEPTH, LAP = CF::LAP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
