@@ -477,3 +477,25 @@ def test_few_shots_of_fp32_blocks_sum_in_fp64(N, S, monkeypatch):
         ur, sr, _ = O.leapfrog(row_ptr, col, rounded, minv, ne, Np, 0.01, 3, 5, phi[k], F[k], [4], phi[:1], u0[k])
         assert rel(u[k], ur) < 1e-12
         assert rel(seis[k], sr) < 1e-12
+
+
+def test_single_shot_rows_in_any_order_at_a_size_line():
+    """Rows whose diagonal block is not the first, at a size whose meshes take
+    the row kernel (which reads u^k from the first block)."""
+    N, ne, Np = 3, 3300, 10
+    row_ptr, col, blocks, minv = random_operator(ne, N, 3, True)
+    order = np.concatenate([np.roll(np.arange(row_ptr[e], row_ptr[e + 1]), e % 3) for e in range(ne)])
+    col, blocks = col[order], blocks[order]
+    rng = np.random.default_rng(7)
+    u0 = rng.standard_normal(2 * ne * Np)
+    phi = rng.standard_normal((1, Np))
+    F = rng.standard_normal((3, 2))
+    with capi.Simulation.from_blocks(row_ptr, col, blocks, minv, [9], phi, [ne - 1], phi) as s:
+        s.set_dt(0.01)
+        s.set_force_table(0, F)
+        s.set_initial(0, u0)
+        s.first_step()
+        s.run(2)
+        u = s.u()
+    ur, _, _ = O.leapfrog(row_ptr, col, blocks, minv, ne, Np, 0.01, 3, 9, phi[0], F, [ne - 1], phi, u0)
+    assert rel(u, ur) < 1e-12

@@ -46,6 +46,7 @@ struct tsp_handle {
   // per face: stored block << 1 | transposed of each pattern entry (empty: the
   // pattern's own order), the rows' references on the device, stored blocks.
   std::vector<int> bref;
+  bool diag_first = true;  // every row begins with its diagonal block (meshes: always)
   tsp::RowRefs* d_rows = nullptr;
   long long nstored = 0;
   int bpitch = 0;  // column pitch of stored blocks: 2Np (one shot) or 2Np rounded up to 4 (batched)
@@ -559,11 +560,14 @@ int rowshots_max(int R, bool fp64, long long ne) {
     default: return 0;
   }
 }
+// The row kernel and the batched kernels take u^k from a row's first block,
+// which is the diagonal one by contract; rows handed over in another order
+// stay with the kernels that look it up by its element.
 bool uses_rowring(const tsp_handle* h) {
   if (h->op_kind != TSP_OP_EXPLICIT || h->prec == TSP_PREC_BF16) return false;
   const bool fp64 = h->prec == TSP_PREC_FP64;
-  if (h->S == 1) return rowring_size(h->R, fp64) && !rowring_slow(h->R, fp64, h->ne);
-  const int most = rowshots_max(h->R, fp64, h->ne);
+  if (h->S == 1) return rowring_size(h->R, fp64) && !(h->diag_first && rowring_slow(h->R, fp64, h->ne));
+  const int most = rowshots_max(h->R, fp64, h->diag_first ? h->ne : 0);
   return rowshots_size(h->R) && h->kernel_variant < 0 && (most == 0 || h->S <= most);
 }
 
@@ -1828,6 +1832,7 @@ int tsp_create_from_blocks(const tsp_block_problem* P, tsp_handle** out) {
   h->nrcv = P->nrcv;
   h->prec = P->precision;
   h->nnzb = P->nnzb;
+  for (int e = 0; e < P->ne; ++e) h->diag_first &= P->col[P->row_ptr[e]] == e;
   if (P->ref_invmass && (rc = set_basis_mass(h, TSP_BASIS_BOUNDARY_ADAPTED, mref, mi))) return create_error_from(h, rc);
   h->src_elem.assign(P->src_elem, P->src_elem + h->S);
   h->src_phi.assign(P->src_phi, P->src_phi + size_t(h->S) * h->Np);
