@@ -499,3 +499,32 @@ def test_single_shot_rows_in_any_order_at_a_size_line():
         u = s.u()
     ur, _, _ = O.leapfrog(row_ptr, col, blocks, minv, ne, Np, 0.01, 3, 9, phi[0], F, [ne - 1], phi, u0)
     assert rel(u, ur) < 1e-12
+
+
+# The row and the ring kernel for FP32 blocks at N = 3 and 4, on both sides of
+# the sizes between them, against the matrix-free operator (bounds as above).
+@pytest.mark.parametrize("N,nx,ny", [(3, 25, 20), (3, 51, 10), (4, 40, 40), (4, 59, 28), (4, 75, 50), (4, 94, 40)])
+def test_fp32_rows_at_the_size_lines(N, nx, ny):
+    m = W.jittered_rect(nx, ny, 100.0 * nx, 100.0 * ny, seed=N)
+    rng = np.random.default_rng(N)
+    vp = 2500 + 1500 * rng.random(m.ne)
+    lam, mu, rho = W.lame(vp, vp / 1.8, 2000 + 500 * rng.random(m.ne))
+    x = rng.standard_normal(m.ne * (N + 1) * (N + 2))
+    out = []
+    for op, prec in (("matrix_free", "fp64"), ("explicit", "fp32")):
+        with capi.Simulation.create(m.xy, m.tri, N, lam, mu, rho, [(40.0, 30.0)], [(61.0, 33.0), (20.0, 55.0)],
+                                    penalty=10.0, op=op, precision=prec) as s:
+            s.set_dt(1e-5)
+            y, lmax = s.apply(x), s.estimate_lmax(10)
+            s.set_ricker(0, 20.0, 0.05, -1e9, 1, 20)
+            s.set_initial(0, 1e-3 * x)
+            s.first_step()
+            s.run(9)
+            out.append((y, s.u(), s.seismograms(0, 10), lmax))
+            stored, nnzb = s.stored_blocks, s.nnzb
+    rows = m.ne > 1000 if N == 3 else 3200 < m.ne <= 7500
+    assert (stored == nnzb) == rows
+    a, b = out
+    for i in range(3):
+        assert rel(b[i], a[i]) < 1e-4
+    assert abs(b[3] - a[3]) < 1e-4 * a[3]

@@ -515,24 +515,29 @@ int upload_rows(tsp_handle* h, const int* row_ptr, const int* col) {
   return TSP_OK;
 }
 
-// Single-shot handles with stored blocks advance by the ring kernel on
-// symmetric storage, FP64 from 2Np = 20 on, FP32 from 2Np = 42 on. Below, a row
-// is so short that the ring kernel's work per row, not its bytes, sets the
-// time, and the register-streaming row kernel wins (40,000 triangles, us per
-// step, ring / rows: FP64 2Np = 12 85 / 37, 20 75 / 84, 30 116 / 327; FP32
-// 2Np = 20 65 / 50, 42 120 / 183; FP32 30: 6,000 triangles 16.1 / 14.4, 40,000
-// 90 / 97). BF16 blocks are not multiples of the 16 bytes
-// of a bulk copy.
-constexpr bool rowring_size(int R, bool fp64) { return R >= (fp64 ? 20 : 42); }
-// FP64 2Np = 20, the smallest rows the ring kernel takes: its step lasts as
-// many rounds as teams (seven per SM) have rows, and between three and twelve
-// thousand triangles the row kernel wins where a round has just begun. us per
-// step, ring / rows, 4 receivers: 2,800 triangles 8.5 / 8.1, 3,200 10.2 / 8.1,
-// 4,000 10.2 / 10.5; 8 receivers: 3,400 10.4 / 9.5, 3,800 10.1 / 11.4, 5,000
-// 11.9 / 13.0, 5,600 14.5 / 13.2, 8,000 17.7 / 16.8, 10,000 21.6 / 20.7, 12,000
-// 25.8 / 25.5, 15,000 31.3 / 38.4.
-constexpr bool rowring_slow(int R, bool fp64, long long ne) {
-  return fp64 && R == 20 && ((ne > 3100 && ne <= 3700) || (ne > 5180 && ne <= 12000));
+// Single-shot handles with stored FP64 or FP32 blocks advance by the ring kernel
+// on symmetric storage or by the register-streaming row kernel on full storage.
+// The ring kernel wins where the bytes of a row outweigh its work per row, at
+// every size from 2Np = 30 FP64 / 42 FP32 on (40,000 triangles, us per step,
+// ring / rows: FP64 2Np = 12 85 / 37, 30 116 / 327; FP32 42 120 / 183). BF16
+// blocks are not multiples of the 16 bytes of a bulk copy.
+constexpr bool rowring_size(int R) { return R >= 20; }
+constexpr bool rowring_always(int R, bool fp64) { return R >= (fp64 ? 30 : 42); }
+// Between, the number of triangles decides: the ring kernel also wins while the
+// teams' rows fit few rounds (short chains, dependent launch), and the row
+// kernel slows down where its full storage leaves L2. us per step, ring / rows:
+//   FP64 20  2,800 triangles 8.5 / 8.1, 3,200 10.2 / 8.1, 4,000 10.2 / 10.5 (4
+//            receivers); 3,400 10.4 / 9.5, 3,800 10.1 / 11.4, 5,000 11.9 / 13.0,
+//            5,600 14.5 / 13.2, 8,000 17.7 / 16.8, 10,000 21.6 / 20.7, 12,000
+//            25.8 / 25.5, 15,000 31.3 / 38.4, 40,000 77 / 84 (8 receivers)
+//   FP32 20  800 4.7 / 6.5, 1,600 7.3 / 6.6, 6,000 14.8 / 9.4, 40,000 82 / 49
+//   FP32 30  800 4.8 / 7.2, 1,600 6.7 / 7.6, 3,200 9.9 / 10.0, 6,000 14.7 / 13.7,
+//            7,000 15.6 (rows), 8,100 18.1 / 20.3, 12,000 27 / 36, 40,000 81 / 91,
+//            160,000 320 / 362
+bool rows_win(int R, bool fp64, long long ne) {
+  if (rowring_always(R, fp64)) return false;
+  if (fp64) return (ne > 3100 && ne <= 3700) || (ne > 5180 && ne <= 12000);
+  return R == 20 ? ne > 1000 : ne > 3200 && ne <= 7500;
 }
 // Handles of a few shots use the same storage with shot tiles of 8 to 32
 // (k_step_rowshots), unless TSP_BATCHED_VARIANT asks for a batched kernel.
@@ -566,7 +571,7 @@ int rowshots_max(int R, bool fp64, long long ne) {
 bool uses_rowring(const tsp_handle* h) {
   if (h->op_kind != TSP_OP_EXPLICIT || h->prec == TSP_PREC_BF16) return false;
   const bool fp64 = h->prec == TSP_PREC_FP64;
-  if (h->S == 1) return rowring_size(h->R, fp64) && !(h->diag_first && rowring_slow(h->R, fp64, h->ne));
+  if (h->S == 1) return rowring_size(h->R) && !(h->diag_first && rows_win(h->R, fp64, h->ne));
   const int most = rowshots_max(h->R, fp64, h->diag_first ? h->ne : 0);
   return rowshots_size(h->R) && h->kernel_variant < 0 && (most == 0 || h->S <= most);
 }
@@ -1184,11 +1189,11 @@ int launch_R(tsp_handle* h, const tsp::StepParams& p, cudaStream_t st) {
   switch (h->prec) {
     case TSP_PREC_FP64:
       if (padded || R % 4 == 0) tsp::k_step_rows<R, double, true><<<grid, RT::THREADS, 0, st>>>(p);
-      else if constexpr (!rowring_size(R, true)) tsp::k_step_rows<R, double, false><<<grid, RT::THREADS, 0, st>>>(p);
+      else if constexpr (!rowring_always(R, true)) tsp::k_step_rows<R, double, false><<<grid, RT::THREADS, 0, st>>>(p);
       break;
     case TSP_PREC_FP32:
       if (padded || R % 4 == 0) tsp::k_step_rows<R, float, true><<<grid, RT::THREADS, 0, st>>>(p);
-      else if constexpr (!rowring_size(R, false)) tsp::k_step_rows<R, float, false><<<grid, RT::THREADS, 0, st>>>(p);
+      else if constexpr (!rowring_always(R, false)) tsp::k_step_rows<R, float, false><<<grid, RT::THREADS, 0, st>>>(p);
       break;
     default:
       if (padded || R % 4 == 0) tsp::k_step_rows<R, __nv_bfloat16, true><<<grid, RT::THREADS, 0, st>>>(p);

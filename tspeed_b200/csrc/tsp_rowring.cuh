@@ -58,8 +58,7 @@ struct alignas(32) RowRefs {
 
 // Bytes of stored blocks from which the rows are claimed instead of shared
 // out: five times L2. us per step at 12,000 triangles, shared out / claimed:
-// FP32 2Np = 72 (0.62 GB) 131 / 132, FP64 56 (0.75 GB) 117 / 112, FP32 90
-// (0.97 GB) 179 / 164.
+// FP64 2Np = 56 (0.75 GB) 114.4 / 113.7, FP32 90 (0.97 GB) 182 / 166.
 constexpr size_t row_queue_bytes = size_t(640) << 20;
 
 template <int R, typename BT>
@@ -74,9 +73,9 @@ struct RowRingCfg {
   // per step (columns, slots, teams): FP64 2Np = 30 (15, 2, 5) 119, (30, 1, 6)
   // 116; 42 (14, 3, 3) 208, (6, 7, 3) 291; 56 (14, 2, 3) 437, (28, 2, 2) 420;
   // 72 (12, 2, 3) 747, (24, 3, 1) 855; 90 (10, 3, 2) 1162, (6, 3, 3) 1313.
-  // FP32 (with lane groups over the columns, before ORD) 42 (42, 2, 3) 122,
-  // (14, 3, 6) 119, (42, 1, 5) 117; 56 (14, 4, 3) 272, (28, 2, 3) 200; 72
-  // (12, 3, 4) 445, (36, 2, 2) 402; 90 (18, 5, 1) 864, (10, 3, 4) 562.
+  // FP32 (columns, slots) 42 (42, 2) 125, (14, 3) 132, (42, 1) 120; 56 (14, 4)
+  // 292, (28, 2) 228; 72 (12, 3) 404, (36, 2) 433 (12,000 triangles 141, 137;
+  // 120,000 1274, 1289); 90 (18, 5) 929, (10, 3) 560.
   static constexpr bool F64 = SZ == 8;
   static constexpr int NC = F64 ? (R == 42 ? 14 : R == 56 ? 28 : R == 72 ? 12 : R == 90 ? 10 : R)
                                 : (R == 56 ? 28 : R == 72 ? 36 : R == 90 ? 10 : R);
@@ -106,10 +105,10 @@ struct RowRingCfg {
   // Rows claimed as teams come free (see the row queue in the kernel), where
   // the blocks are of several times the size of L2 (row_queue_bytes). us per
   // step with a fixed share of rows / claimed, 40,000 triangles: FP64 2Np = 56
-  // 430 / 367, 72 752 / 631; FP32 56 242 / 226, 72 448 / 429, 90 718 / 552;
-  // 120,000 triangles: FP64 56 1439 / 1133, 72 2650 / 2089, FP32 56 799 / 669,
-  // 90 2335 / 1809. Smaller rows lose: FP64 30 115 / 157, 42 211 / 221, FP32
-  // 42 118 / 118.
+  // 414 / 362, 72 773 / 634; FP32 56 245 / 228, 72 451 / 433, 90 721 / 560;
+  // 120,000 triangles: FP64 56 1495 / 1164, 72 2632 / 2084, FP32 56 800 / 687,
+  // 72 1396 / 1289. Smaller rows lose: FP64 30 115 / 157, 42 211 / 221, FP32
+  // 42 118 / 118 (before FP32 sums went in column order).
   static constexpr bool QUEUE = R >= 56;
   static constexpr int LOOK = DEPTH + 2;
   static constexpr int CLAIM = LOOK + 4;
