@@ -938,6 +938,7 @@ std::vector<double> matfree_lean_tables(const tsp::RefTables& T) {
 bool matfree_lean(tsp_handle* h, int Q, int degrees) {
   if (degrees >= 3 && h->ne > 200 && h->ne <= 1000) return true;
   const size_t kept = size_t(h->ne) * (46 + 2 * 3 * size_t(Q) * 4) * sizeof(double);
+  if (kept < (size_t(32) << 20)) return false;  // asking takes 0.08 ms, a sixth of a small handle's creation
   size_t room = 0, total = 0;
   if (cudaMemGetInfo(&room, &total) != cudaSuccess) {
     cudaGetLastError();
