@@ -20,7 +20,7 @@
 // step with one warp per element on the CUDA cores (neighbours' traces
 // recomputed, tables read element by element) / now: 160,000 triangles N = 6
 // 1146 / 249; 40,000 triangles N = 4 153 / 32, N = 8 579 / 169; 6,734 triangles
-// N = 3 24.9 / 7.9. Bound: the FP64 tensor rate (478 MMAs per tile at N = 6:
+// N = 3 24.9 / 7.5. Bound: the FP64 tensor rate (478 MMAs per tile at N = 6:
 // 132 us for 160,000 triangles; the pipe is busy half of the time) and the
 // latency of a tile's loads, of which
 // two rounds are left: what a tile starts with (face records, neighbours,
