@@ -2297,7 +2297,7 @@ int tsp_get_state(tsp_handle* h, double* u_prev, double* u_cur, int64_t* steps_d
   }
   if (steps_done) *steps_done = h->steps_done;
   if (last_time) *last_time = h->last_time;
-  return check_device_error(h);
+  return u_prev || u_cur ? check_device_error(h) : TSP_OK;  // without a level nothing was waited for
 }
 
 int tsp_set_state(tsp_handle* h, const double* u_prev, const double* u_cur, int64_t steps_done, double last_time) {
